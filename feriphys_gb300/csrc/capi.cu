@@ -300,10 +300,10 @@ int ensure_topology(fgb_mesh* m) {
   free_topology(m);
   FGB_CHECK_RC(decide_path(m, &m->active_path));
   if (m->active_path == 2) {
-    std::vector<float> planes;
-    fgb::build_grid_params(m->topo, planes);
-    FGB_CUDA(dalloc(m->d_grid, planes.size() * sizeof(float)));
-    FGB_CUDA(cudaMemcpy(m->d_grid, planes.data(), planes.size() * sizeof(float), cudaMemcpyHostToDevice));
+    std::vector<float> params;
+    fgb::build_grid_params(m->topo, params);
+    FGB_CUDA(dalloc(m->d_grid, params.size() * sizeof(float)));
+    FGB_CUDA(cudaMemcpy(m->d_grid, params.data(), params.size() * sizeof(float), cudaMemcpyHostToDevice));
   } else {
     FGB_CHECK_RC(ensure_csr(m));
   }
@@ -428,7 +428,7 @@ int prepare_batch(fgb_sim* s) {
     fgb_mesh* m = grid[i];
     fgb::ClothDesc& d = desc[i];
     std::memset(&d, 0, sizeof(d));
-    d.planes = m->d_grid;
+    d.params = m->d_grid;
     for (int k = 0; k < 2; ++k) {
       d.pos[k] = static_cast<float4*>(m->pos[k]);
       d.vel[k] = static_cast<float4*>(m->vel[k]);
@@ -455,7 +455,6 @@ int prepare_batch(fgb_sim* s) {
     FGB_CUDA(cudaMemcpy(s->d_work, work.data(), work.size() * sizeof(int), cudaMemcpyHostToDevice));
     s->n_work = int(work.size() / 4);
     s->work_host = work;
-    if (!s->d_counter) FGB_CUDA(dalloc(s->d_counter, sizeof(int)));
     if (membership) s->mode = -1;
   }
   if (membership || reshape || desc.size() != s->desc.size() ||
@@ -468,25 +467,6 @@ int prepare_batch(fgb_sim* s) {
     }
     FGB_CUDA(cudaMemcpyAsync(s->d_desc, desc.data(), desc.size() * sizeof(fgb::ClothDesc), cudaMemcpyHostToDevice,
                              bs));
-    // TMA staging maps for every cloth's buffers (all or none)
-    std::vector<unsigned char> maps(desc.size() * fgb::kClothMapBytes + 64);
-    unsigned char* mp = maps.data() + ((64 - (reinterpret_cast<uintptr_t>(maps.data()) & 63)) & 63);
-    bool maps_ok = true;
-    for (size_t i = 0; i < desc.size() && maps_ok; ++i)
-      maps_ok = fgb::encode_cloth_maps(desc[i], s->tile_h, mp + i * fgb::kClothMapBytes);
-    if (maps_ok) {
-      if (s->d_maps_cap < desc.size() || !s->d_maps) {
-        drop_graphs(s);
-        s->d_maps_cap = 0;
-        FGB_CUDA(dalloc(s->d_maps, desc.size() * fgb::kClothMapBytes));
-        s->d_maps_cap = desc.size();
-      }
-      FGB_CUDA(cudaMemcpyAsync(s->d_maps, mp, desc.size() * fgb::kClothMapBytes, cudaMemcpyHostToDevice, bs));
-    } else {
-      dfree(s->d_maps);
-      s->d_maps_cap = 0;
-      drop_graphs(s);
-    }
     FGB_CUDA(cudaStreamSynchronize(bs));
     s->desc = std::move(desc);
   }
@@ -495,33 +475,30 @@ int prepare_batch(fgb_sim* s) {
   return FGB_OK;
 }
 
-int batch_launch(fgb_sim* s, int parity, int mode, int ctas) {
-  cudaStream_t st = batch_stream(s);
-  FGB_CUDA(cudaMemsetAsync(s->d_counter, 0, sizeof(int), st));
-  FGB_CUDA(fgb::launch_step_batched(s->d_desc, s->d_work, s->n_work, s->d_counter, parity, mode, ctas,
-                                    make_consts(s->cfg, s->d_faces, s->n_faces, nullptr, &s->accel), st, s->d_maps,
+int batch_launch(fgb_sim* s, int parity) {
+  FGB_CUDA(fgb::launch_step_batched(s->d_desc, s->d_work, s->n_work, parity,
+                                    make_consts(s->cfg, s->d_faces, s->n_faces, nullptr, &s->accel), batch_stream(s),
                                     nullptr, s->tile_h));
   return FGB_OK;
 }
 
 // Autotuner: times every tile height (32 x 4, 32 x 8, 32 x 12 vertex tiles,
-// each with its own block size) and launch form (one CTA per tile, or
-// persistent CTAs at the occupancy the tile allows) on this batch -- launches
-// that read the current buffers and write the other ones, so the state is
-// untouched -- and caches the winner per GPU and batch in a text file
-// ($FGB_AUTOTUNE_CACHE, default ~/.cache/feriphys_gb300/autotune.txt).
+// each with its own block size) on this batch -- launches that read the
+// current buffers and write the other ones, so the state is untouched -- and
+// caches the winner per GPU and batch in a text file ($FGB_AUTOTUNE_CACHE,
+// default ~/.cache/feriphys_gb300/autotune.txt).
 std::string tune_cache_path() {
   if (const char* p = std::getenv("FGB_AUTOTUNE_CACHE")) return p;
   const char* home = std::getenv("HOME");
   return std::string(home ? home : "/tmp") + "/.cache/feriphys_gb300/autotune.txt";
 }
 
-int use_launch_form(fgb_sim* s, int tile_h, int mode, int sms) {
+int use_tile(fgb_sim* s, int tile_h, int sms) {
   if (s->tile_h != tile_h) {
     s->tile_h = tile_h;
-    FGB_CHECK_RC(prepare_batch(s));  // work list and maps for this tile height
+    FGB_CHECK_RC(prepare_batch(s));  // work list for this tile height
   }
-  s->mode = mode;
+  s->mode = s->forced_mode > 0 ? s->forced_mode : 0;
   s->ctas = fgb::batched_ctas_per_sm(tile_h) * sms;
   return FGB_OK;
 }
@@ -532,42 +509,33 @@ int tune_batch(fgb_sim* s) {
   cudaDeviceProp prop;
   FGB_CUDA(cudaGetDeviceProperties(&prop, dev));
   const int sms = prop.multiProcessorCount;
-  std::vector<int> heights, modes;
-  if (s->forced_tile_h > 0) heights.push_back(s->forced_tile_h);
-  else heights.assign(std::begin(fgb::kBatchTileHeights), std::end(fgb::kBatchTileHeights));
-  if (s->forced_mode >= 0) modes.push_back(s->forced_mode);
-  else modes = {0, 1};
-  if (heights.size() == 1 && modes.size() == 1) return use_launch_form(s, heights[0], modes[0], sms);
+  if (s->forced_tile_h > 0) return use_tile(s, s->forced_tile_h, sms);
+  const std::vector<int> heights(std::begin(fgb::kBatchTileHeights), std::end(fgb::kBatchTileHeights));
   size_t verts = 0;
   for (const fgb_mesh* m : s->batch) verts += m->topo.n;
   int vb = 0, cb = 0;
   while ((size_t(1) << vb) < verts) ++vb;
   while ((size_t(1) << cb) < s->batch.size()) ++cb;
   char key[512];
-  std::snprintf(key, sizeof(key), "batched %s sms=%d cloths=2^%d vertices=2^%d heights=%zu modes=%zu", prop.name, sms,
-                cb, vb, heights.size(), modes.size());
+  std::snprintf(key, sizeof(key), "batched pairs %s sms=%d cloths=2^%d vertices=2^%d heights=%zu", prop.name, sms, cb,
+                vb, heights.size());
   for (char* c = key; *c; ++c)
     if (*c == '\n') *c = ' ';
   const std::string path = tune_cache_path();
   if (FILE* f = std::fopen(path.c_str(), "r")) {
     char line[600];
-    int mode = -1, th = 0;
+    int th = 0;
     while (std::fgets(line, sizeof(line), f)) {
-      int m = -1, t = 0;
+      int t = 0;
       const char* sep = std::strstr(line, " -> ");
       if (!sep || std::string(line, sep - line) != key) continue;
-      if (std::sscanf(sep + 4, "mode=%d tile_h=%d", &m, &t) == 2 && (m == 0 || m == 1) &&
-          fgb::batch_tile_height_ok(t) && std::find(heights.begin(), heights.end(), t) != heights.end() &&
-          std::find(modes.begin(), modes.end(), m) != modes.end()) {
-        mode = m;
-        th = t;
-      }
+      if (std::sscanf(sep + 4, "tile_h=%d", &t) == 1 && fgb::batch_tile_height_ok(t)) th = t;
     }
     std::fclose(f);
-    if (mode >= 0) return use_launch_form(s, th, mode, sms);
+    if (th > 0) return use_tile(s, th, sms);
   }
   float best = 1e30f;
-  int best_mode = modes[0], best_h = heights[0];
+  int best_h = heights[0];
   cudaEvent_t a, b;
   FGB_CUDA(cudaEventCreate(&a));
   if (const cudaError_t e = cudaEventCreate(&b); e != cudaSuccess) {
@@ -576,29 +544,25 @@ int tune_batch(fgb_sim* s) {
   }
   int rc = FGB_OK;
   for (int th : heights) {
-    for (int mode : modes) {
-      if ((rc = use_launch_form(s, th, mode, sms)) != FGB_OK) break;
-      if ((rc = batch_launch(s, s->parity, mode, s->ctas)) != FGB_OK) break;  // warm-up
-      cudaEventRecord(a, batch_stream(s));
-      for (int r = 0; r < 5 && rc == FGB_OK; ++r) rc = batch_launch(s, s->parity, mode, s->ctas);
-      cudaEventRecord(b, batch_stream(s));
-      float ms = 0.0f;
-      cudaError_t e = cudaEventSynchronize(b);
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
-      if (rc == FGB_OK && e != cudaSuccess) rc = fail(FGB_ECUDA, cudaGetErrorString(e));
-      if (rc != FGB_OK) break;
-      if (ms < best) {
-        best = ms;
-        best_mode = mode;
-        best_h = th;
-      }
-    }
+    if ((rc = use_tile(s, th, sms)) != FGB_OK) break;
+    if ((rc = batch_launch(s, s->parity)) != FGB_OK) break;  // warm-up
+    cudaEventRecord(a, batch_stream(s));
+    for (int r = 0; r < 5 && rc == FGB_OK; ++r) rc = batch_launch(s, s->parity);
+    cudaEventRecord(b, batch_stream(s));
+    float ms = 0.0f;
+    cudaError_t e = cudaEventSynchronize(b);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
+    if (rc == FGB_OK && e != cudaSuccess) rc = fail(FGB_ECUDA, cudaGetErrorString(e));
     if (rc != FGB_OK) break;
+    if (ms < best) {
+      best = ms;
+      best_h = th;
+    }
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   if (rc != FGB_OK) return rc;
-  FGB_CHECK_RC(use_launch_form(s, best_h, best_mode, sms));
+  FGB_CHECK_RC(use_tile(s, best_h, sms));
   const std::string dir = path.substr(0, path.rfind('/'));
   // create the cache directory (best effort) and append the result
   for (size_t i = 1; i <= dir.size(); ++i)
@@ -607,8 +571,7 @@ int tune_batch(fgb_sim* s) {
       mkdir(sub.c_str(), 0755);
     }
   if (FILE* f = std::fopen(path.c_str(), "a")) {
-    std::fprintf(f, "%s -> mode=%d tile_h=%d ctas_per_sm=%d time_ms=%.4f\n", key, best_mode, best_h,
-                 s->ctas / sms, best / 5.0f);
+    std::fprintf(f, "%s -> tile_h=%d ctas_per_sm=%d time_ms=%.4f\n", key, best_h, s->ctas / sms, best / 5.0f);
     std::fclose(f);
   }
   return FGB_OK;
@@ -621,7 +584,7 @@ int batched_steps(fgb_sim* s, uint64_t n) {
   for (fgb_mesh* m : s->batch) forces = forces || m->has_force;
   if (forces) {  // the first step carries accumulated forces: run it directly
     if (s->mode < 0) FGB_CHECK_RC(tune_batch(s));
-    FGB_CHECK_RC(batch_launch(s, s->parity, s->mode, s->ctas));
+    FGB_CHECK_RC(batch_launch(s, s->parity));
     s->parity ^= 1;
     for (fgb_mesh* m : s->batch) {
       m->cur = s->parity;
@@ -644,7 +607,7 @@ int batched_steps(fgb_sim* s, uint64_t n) {
       cudaGraph_t g;
       FGB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       int rc = FGB_OK;
-      for (uint64_t k = 0; k < n && rc == FGB_OK; ++k) rc = batch_launch(s, s->parity ^ int(k & 1), s->mode, s->ctas);
+      for (uint64_t k = 0; k < n && rc == FGB_OK; ++k) rc = batch_launch(s, s->parity ^ int(k & 1));
       const cudaError_t e = cudaStreamEndCapture(st, &g);
       if (rc != FGB_OK) return rc;
       FGB_CUDA(e);
@@ -656,7 +619,7 @@ int batched_steps(fgb_sim* s, uint64_t n) {
     }
     FGB_CUDA(cudaGraphLaunch(it->second, st));
   } else {
-    for (uint64_t k = 0; k < n; ++k) FGB_CHECK_RC(batch_launch(s, s->parity ^ int(k & 1), s->mode, s->ctas));
+    for (uint64_t k = 0; k < n; ++k) FGB_CHECK_RC(batch_launch(s, s->parity ^ int(k & 1)));
   }
   s->parity ^= int(n & 1);
   for (fgb_mesh* m : s->batch) {
@@ -712,6 +675,31 @@ int upload_faces(fgb_sim* s) {
       s->accel.always = s->d_accel + n_off + n_cf;
       s->accel.grids = reinterpret_cast<const fgb::ObsGrid3*>(s->d_accel + gofs);
       s->accel.n_grids = int(a.grids.size());
+      s->accel.n_boxes = 0;
+      for (const fgb::ObsGrid3& g : a.grids) {
+        fgb::ObsBox b{};
+        const bool all = g.n_always != 0;
+        if (!all && g.n[0] <= 0) continue;  // no face of this obstacle can be hit
+        for (int d = 0; d < 3; ++d) {
+          b.lo[d] = all ? -INFINITY : g.lo[d];
+          b.hi[d] = all ? INFINITY : g.hi[d];
+          b.cell[d] = g.cell[d];
+          b.inv[d] = g.inv[d];
+          b.n[d] = all ? 0 : g.n[d];
+        }
+        b.slack = g.slack;
+        b.off_base = g.off_base;
+        if (s->accel.n_boxes < fgb::kObsBoxes) {
+          s->accel.box[s->accel.n_boxes++] = b;
+          continue;
+        }
+        fgb::ObsBox& u = s->accel.box[fgb::kObsBoxes - 1];
+        for (int d = 0; d < 3; ++d) {
+          u.lo[d] = std::min(u.lo[d], b.lo[d]);
+          u.hi[d] = std::max(u.hi[d], b.hi[d]);
+          u.n[d] = 0;
+        }
+      }
     }
     s->faces_uploaded = true;
   }
@@ -1358,8 +1346,6 @@ int fgb_sim_destroy(fgb_sim* s) {
   for (auto& kv : s->graph_cache) cudaGraphExecDestroy(kv.second);
   dfree(s->d_desc);
   dfree(s->d_work);
-  dfree(s->d_counter);
-  dfree(s->d_maps);
   delete s;
   return FGB_OK;
 }
@@ -1391,9 +1377,8 @@ cudaStream_t fgb::detail::sim_stream(fgb_sim* s) {
 // their own allocators and forbid plugin allocations inside the frame loop,
 // and real-time loops that cannot afford cudaMalloc/cudaFree (both can
 // synchronise the whole device).  fgb_sim_step_static advances a prepared
-// simulation with the batched persistent kernel while keeping that kernel's
-// scratch -- its work counter, the cloth descriptor table and the tile list --
-// in the fixed array below instead of memory allocated for the simulation.
+// simulation with the batched kernel while keeping that kernel's scratch -- the
+// cloth descriptor table and the tile list -- in the fixed array below instead of memory allocated for the simulation.
 
 namespace {
 
@@ -1481,7 +1466,7 @@ extern "C" int fgb_sim_step_static(fgb_sim* s, uint64_t n_steps, void* stream) {
     fgb_mesh* m = order[i];
     fgb::ClothDesc& d = desc[i];
     std::memset(&d, 0, sizeof(d));
-    d.planes = m->d_grid;
+    d.params = m->d_grid;
     for (int k = 0; k < 2; ++k) {
       d.pos[k] = static_cast<float4*>(m->pos[k]);
       d.vel[k] = static_cast<float4*>(m->vel[k]);
@@ -1494,18 +1479,11 @@ extern "C" int fgb_sim_step_static(fgb_sim* s, uint64_t n_steps, void* stream) {
   }
   fgb::ClothDesc* d_desc = reinterpret_cast<fgb::ClothDesc*>(scratch + desc_off);
   int4* d_work = reinterpret_cast<int4*>(scratch + work_off);
-  int* d_counter = reinterpret_cast<int*>(scratch);
   FGB_CUDA(cudaMemcpyAsync(d_desc, desc.data(), desc.size() * sizeof(fgb::ClothDesc), cudaMemcpyHostToDevice, st));
   FGB_CUDA(cudaMemcpyAsync(d_work, work.data(), work.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-  int dev = 0, sms = 0;
-  FGB_CUDA(cudaGetDevice(&dev));
-  FGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int ctas = fgb::batched_ctas_per_sm() * sms;
   s->accel.enabled = (s->broadphase && s->d_accel) ? 1 : 0;
   for (uint64_t k = 0; k < n_steps; ++k) {
-    // the counter keeps the previous call's value: clear it before every launch
-    FGB_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
-    FGB_CUDA(fgb::launch_step_batched(d_desc, d_work, int(n_work), d_counter, int(k & 1), 1, ctas,
+    FGB_CUDA(fgb::launch_step_batched(d_desc, d_work, int(n_work), int(k & 1),
                                       make_consts(s->cfg, s->d_faces, s->n_faces, nullptr, &s->accel), st));
     if (k == 0 && n_steps > 1) {  // carried forces apply to the first step only
       bool forces = false;

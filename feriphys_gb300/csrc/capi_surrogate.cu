@@ -97,7 +97,6 @@ struct fgb_surrogate {
   size_t fdesc_cap = 0;
   int4* d_fwork = nullptr;            // work items of the failing cloths only
   size_t fwork_cap = 0;
-  int* d_fcounter = nullptr;
   int groups = 4;
   // checked rollout decided on the device (per cloth: accepted energy, margin
   // scale, verdict; per batch cloth: work-list range, mesh index, compacted
@@ -272,7 +271,7 @@ S::SurCloth make_cloth(fgb_mesh* m, float T, const float wind[3], long long vbas
     c.pos[k] = static_cast<float4*>(m->pos[k]);
     c.vel[k] = static_cast<float4*>(m->vel[k]);
   }
-  c.planes = m->d_grid;
+  c.params = m->d_grid;
   c.rest = m->d_rest;
   c.flags = m->d_flags;
   c.rows = int(m->topo.rows);
@@ -400,7 +399,6 @@ int fine_fallback(fgb_surrogate* g, fgb_sim* s, const std::vector<int>& failing,
   const int n_fw = int(fw.size() / 4);
   FGB_CUDA(dgrow(g->d_fdesc, g->fdesc_cap, d.size(), sizeof(fgb::ClothDesc)));
   FGB_CUDA(dgrow(g->d_fwork, g->fwork_cap, std::max<size_t>(fw.size() / 4, 1), sizeof(int4)));
-  if (!g->d_fcounter) FGB_CUDA(cudaMalloc(&g->d_fcounter, sizeof(int)));
   FGB_CUDA(cudaMemcpyAsync(g->d_fdesc, d.data(), d.size() * sizeof(fgb::ClothDesc), cudaMemcpyHostToDevice, st));
   if (n_fw) FGB_CUDA(cudaMemcpyAsync(g->d_fwork, fw.data(), fw.size() * sizeof(int), cudaMemcpyHostToDevice, st));
   int from = par;
@@ -408,19 +406,8 @@ int fine_fallback(fgb_surrogate* g, fgb_sim* s, const std::vector<int>& failing,
     FGB_CUDA(S::launch_copy_unskipped(g->d_fdesc, int(d.size()), par, st));
     from = par ^ 1;
   }
-  int ctas = s->ctas;
-  if (s->mode != 1 || ctas <= 0) {
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ctas = fgb::batched_ctas_per_sm(s->tile_h) * sms;
-  }
-  ctas = std::max(1, std::min(ctas, n_fw));
-  for (uint32_t j = 0; j < ratio && n_fw > 0; ++j) {
-    FGB_CUDA(cudaMemsetAsync(g->d_fcounter, 0, sizeof(int), st));
-    FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, n_fw, g->d_fcounter, from ^ int(j & 1u), 1, ctas, fc,
-                                      st, s->d_maps, nullptr, s->tile_h));
-  }
+  for (uint32_t j = 0; j < ratio && n_fw > 0; ++j)
+    FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, n_fw, from ^ int(j & 1u), fc, st, nullptr, s->tile_h));
   FGB_CUDA(cudaStreamSynchronize(st));  // the host table must outlive its upload
   return FGB_OK;
 }
@@ -432,7 +419,7 @@ constexpr int kHostDecides = 1;  // not an error: run the host-decided loop inst
 // Inputs of the graph-built rollout that stay fixed for one call.
 struct Rollout {
   uint32_t ratio = 1;
-  int n_tiles = 0, n_cloths = 0, n_batch = 0, ctas = 1;
+  int n_tiles = 0, n_cloths = 0, n_batch = 0;
   fgb::StepConsts coarse, fine;
   float3 gforce;
   float growth = 0.0f, abs_margin = 0.0f, max_strain = 0.0f;
@@ -471,11 +458,9 @@ int capture_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, c
       FGB_CUDA(S::launch_copy_unskipped(g->d_fdesc, nb, par, bs));
       from = par ^ 1;
     }
-    for (uint32_t j = 0; j < ro.ratio; ++j) {
-      FGB_CUDA(cudaMemsetAsync(g->d_fcounter, 0, sizeof(int), bs));
-      FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, s->n_work, g->d_fcounter, from ^ int(j & 1u), 1,
-                                        ro.ctas, ro.fine, bs, s->d_maps, g->d_counts + 1, s->tile_h));
-    }
+    for (uint32_t j = 0; j < ro.ratio; ++j)
+      FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, s->n_work, from ^ int(j & 1u), ro.fine, bs,
+                                        g->d_counts + 1, s->tile_h));
   }
   FGB_CUDA(S::launch_check(g->d_cloths, g->d_tiles, ro.n_tiles, ro.n_cloths, par ^ 1, ro.gforce, g->d_tile_chk,
                            g->d_cloth_chk, bs));
@@ -588,19 +573,10 @@ int rollout_on_device(fgb_surrogate* g, fgb_sim* s, uint32_t ratio, uint64_t n_c
       if (mi >= s->meshes.size()) return kHostDecides;
       bidx[2 * nb + b] = int(mi);
     }
-    int ctas = s->ctas;
-    if (s->mode != 1 || ctas <= 0) {
-      int dev = 0, sms = 1;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      ctas = fgb::batched_ctas_per_sm(s->tile_h) * sms;
-    }
-    ro.ctas = std::max(1, std::min(ctas, s->n_work));
     FGB_CUDA(dgrow(g->d_bidx, g->bidx_cap, bidx.size(), sizeof(int)));
     FGB_CUDA(dgrow(g->d_fdesc, g->fdesc_cap, size_t(nb), sizeof(fgb::ClothDesc)));
     FGB_CUDA(dgrow(g->d_fwork, g->fwork_cap, size_t(std::max(s->n_work, 1)), sizeof(int4)));
-    if (!g->d_fcounter) FGB_CUDA(cudaMalloc(&g->d_fcounter, sizeof(int)));
-  }
+    }
   FGB_CUDA(dgrow(g->d_e_old, g->e_old_cap, size_t(nc), sizeof(float)));
   FGB_CUDA(dgrow(g->d_e_ref, g->e_ref_cap, size_t(nc), sizeof(double)));
   FGB_CUDA(dgrow(g->d_fail, g->fail_cap, size_t(nc), sizeof(int)));
@@ -728,7 +704,6 @@ int fgb_surrogate_destroy(fgb_surrogate* g) {
   dfree(g->d_out);
   dfree(g->d_fdesc);
   dfree(g->d_fwork);
-  dfree(g->d_fcounter);
   dfree(g->d_e_old);
   dfree(g->d_e_ref);
   dfree(g->d_fail);

@@ -17,6 +17,8 @@
 // vertex, a shear strut (i+1, i+C) by its quad origin i.
 #pragma once
 
+#include <stddef.h>
+
 #if defined(__CUDACC__)
 #define FGB_HD __host__ __device__ __forceinline__
 #else
@@ -97,12 +99,25 @@ FGB_HD FaceDesc face_desc(int s) {
 
 FGB_HD bool quad_exists(int r, int c, int R, int C) { return r >= 0 && c >= 0 && r <= R - 2 && c <= C - 2; }
 
-// Parameter plane layout: 4 float4 per vertex, 15 used floats.
-//   plane 0: kH  cH  LH  kV
-//   plane 1: cV  LV  kS  cS
-//   plane 2: LS  kBH cBH LBH
-//   plane 3: kBV cBV LBV -
-FGB_HD int param_index(int kind, int field /*0 k, 1 c, 2 L*/) { return 3 * kind + field; }
+// Strut constants: one record of kParamRec floats per grid row and block of
+// 32 columns, the columns pc and pc + 16 of the block side by side as the two
+// lanes of the tiled kernel's arithmetic:
+//   [64 kind + 4 pc + 0, 1]   k of columns pc, pc + 16
+//   [64 kind + 4 pc + 2, 3]   c
+//   [320 + 32 kind + 2 pc + 0, 1]   L
+// then, the same way (4 j at kParamLeft for k and c, 2 j at kParamLeft + 16
+// for L), what the tile needs of the columns left of each lane: j = 0, 1 the
+// horizontal and the shear strut of columns -1 | 15, j = 2, 3 the horizontal
+// binding struts of columns -2 | 14 and -1 | 15 (lane 0's are copies of the
+// block to the left's).  Struts that do not exist, and the columns that fill
+// up the last block, have zeros.
+constexpr int kParamLeft = 480, kParamRec = 504;
+FGB_HD size_t param_rec(int r, int c, int C) { return (size_t(r) * ((C + 31) / 32) + c / 32) * kParamRec; }
+FGB_HD size_t param_at(int kind, int field /*0 k, 1 c, 2 L*/, int r, int c, int C) {
+  const int pc = c % 16, lane = (c / 16) % 2;
+  return param_rec(r, c, C) + (field < 2 ? 64 * kind + 4 * pc + 2 * field + lane : 320 + 32 * kind + 2 * pc + lane);
+}
+inline size_t param_count(int R, int C) { return size_t(R) * ((C + 31) / 32) * kParamRec; }
 
 }  // namespace grid
 }  // namespace fgb

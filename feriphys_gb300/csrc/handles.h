@@ -89,7 +89,7 @@ struct fgb_mesh {
   uint16_t* d_face_word = nullptr;
   int compact_form = 0;  // 0 none, 1 32-bit strut words, 2 16-bit strut words
   // grid topology
-  float4* d_grid = nullptr;
+  float* d_grid = nullptr;
   float4* d_rest = nullptr;  // construction positions (x, y, z, 0), uploaded for the surrogate's inputs
 
   size_t elem() const { return precision == 64 ? sizeof(fgb::Dbl4) : sizeof(float4); }
@@ -114,15 +114,12 @@ struct fgb_sim {
   int4* d_work = nullptr;
   int n_work = 0;
   std::vector<int> work_host;             // host copy of the work list (4 ints per item)
-  unsigned char* d_maps = nullptr;        // per batch cloth: 4 tensor maps for TMA staging (null: thread staging)
-  size_t d_maps_cap = 0;
-  int* d_counter = nullptr;
   int parity = 0;
-  int mode = -1, ctas = 0;                // launch form chosen by the tuner
-  int forced_mode = -1;                   // fgb_sim_set_batch_mode (-1: tuner)
+  int mode = -1, ctas = 0;                // launch form (-1: not tuned yet), CTAs resident at once
+  int forced_mode = -1;                   // fgb_sim_set_batch_mode
   int tile_h = fgb::kDefaultTileH;        // tile height (rows) chosen by the tuner
   int forced_tile_h = 0;                  // fgb_sim_set_batch_tile (0: tuner)
-  int built_tile_h = -1;                  // tile height of the uploaded work list and maps
+  int built_tile_h = -1;                  // tile height of the uploaded work list
   bool graphs = true;
   std::map<std::pair<uint64_t, int>, cudaGraphExec_t> graph_cache;
   fgb_config graph_cfg;

@@ -30,10 +30,10 @@ struct GeneralTopo {
 };
 
 // Grid (Cloth::new topology) description for the stencil kernel (see
-// step_grid.cu).  params holds 4 planes of n float4 (owned-strut constants).
+// step_grid.cu).  params holds the strut constants (grid_order.h: param_rec).
 struct GridTopo {
   int rows, cols;
-  const float4* params;
+  const float* params;
   int variant;  // 0: shared-memory tiles, 1: one thread per vertex reading global memory
 };
 
@@ -58,7 +58,7 @@ cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4*
 // One cloth of a batch (Cloth::new topology); buffers [parity] are read and
 // [parity ^ 1] written by a step.
 struct ClothDesc {
-  const float4* planes;
+  const float* params;  // strut constants (grid_order.h: param_rec)
   float4* pos[2];
   float4* vel[2];
   const float4* force_in;  // accumulated force carried into the step, or null
@@ -82,24 +82,15 @@ void batch_tiles(int cloth, int rows, int cols, int th, int* out4 /* may be null
 // in blockIdx order, by the kernel's own mapping.
 int grid_tiles(int rows, int cols, int th, int* out3 /* may be null */);
 
-// mode 0: one CTA per work item; mode 1: persistent CTAs pulling items from
-// *counter (reset to 0 by the caller before the launch).
-// maps: null, or per cloth 4 tensor maps {pos[0], vel[0], pos[1], vel[1]}
-// (encode_cloth_maps) for TMA staging of the tiles.  n_work_dev: null, or the
-// item count in device memory (mode 1 only; n_work is then its upper bound,
-// which sizes the grid).
-// th: the tile height the work list and the maps were made for.
-cudaError_t launch_step_batched(const ClothDesc* cloths, const int4* work, int n_work, int* counter, int parity,
-                                int mode, int persistent_ctas, const StepConsts& c, cudaStream_t s,
-                                const void* maps = nullptr, const int* n_work_dev = nullptr,
+// One CTA per work item.  n_work_dev: null, or the item count in device memory
+// (n_work is then its upper bound, which sizes the grid).
+// th: the tile height the work list was made for.
+cudaError_t launch_step_batched(const ClothDesc* cloths, const int4* work, int n_work, int parity,
+                                const StepConsts& c, cudaStream_t s, const int* n_work_dev = nullptr,
                                 int th = kDefaultTileH);
 // Sets the launch attributes of the tiled and batched step kernels (done by
 // their launchers on first use; call it before a stream capture).
 cudaError_t prime_step_kernels();
-// Size of one cloth's tensor maps (4 x 128 bytes) and their encoding; false
-// when the driver's encoder is unavailable or an address is misaligned.
-constexpr size_t kClothMapBytes = 4 * 128;
-bool encode_cloth_maps(const ClothDesc& d, int th, void* out /* kClothMapBytes, 64-byte aligned */);
 int batched_ctas_per_sm(int th = kDefaultTileH);
 
 }  // namespace fgb

@@ -507,9 +507,9 @@ bool grid_layout_ok(const MeshTopo& m) {
   return true;
 }
 
-void build_grid_params(const MeshTopo& m, std::vector<float>& planes) {
-  const uint32_t n = m.n, C = m.cols;
-  planes.assign(16 * size_t(n), 0.0f);
+void build_grid_params(const MeshTopo& m, std::vector<float>& params) {
+  const uint32_t C = m.cols;
+  params.assign(grid::param_count(int(m.rows), int(C)), 0.0f);
   for (size_t s = 0; s < m.sa.size(); ++s) {
     const uint32_t a = m.sa[s], b = m.sb[s];
     int kind;
@@ -528,11 +528,23 @@ void build_grid_params(const MeshTopo& m, std::vector<float>& planes) {
       owner = a - 1;
     }
     const float vals[3] = {m.sk[s], m.sc[s], m.sl[s]};
-    for (int f = 0; f < 3; ++f) {
-      const int slot = grid::param_index(kind, f);  // 0..14
-      planes[size_t(slot / 4) * 4 * n + 4 * size_t(owner) + size_t(slot % 4)] = vals[f];
-    }
+    for (int f = 0; f < 3; ++f)
+      params[grid::param_at(kind, f, int(owner / C), int(owner % C), int(C))] = vals[f];
   }
+  // the copies for the columns left of each lane
+  const int left_kind[4] = {grid::KH, grid::KS, grid::KBH, grid::KBH}, left_col[4] = {-1, -1, -2, -1};
+  const int R = int(m.rows), nb = (int(C) + 31) / 32;
+  for (int r = 0; r < R; ++r)
+    for (int b = 0; b < nb; ++b) {
+      float* rec = params.data() + grid::param_rec(r, 32 * b, int(C)) + grid::kParamLeft;
+      for (int j = 0; j < 4; ++j)
+        for (int lane = 0; lane < 2; ++lane) {
+          const int c = 32 * b + 16 * lane + left_col[j];
+          if (c < 0 || c >= int(C)) continue;
+          for (int f = 0; f < 3; ++f)
+            rec[f < 2 ? 4 * j + 2 * f + lane : 16 + 2 * j + lane] = params[grid::param_at(left_kind[j], f, r, c, int(C))];
+        }
+    }
 }
 
 }  // namespace fgb

@@ -2,7 +2,7 @@
 // (SpringyMesh::new springy_mesh.rs:267-401, add_strut 403-413, add_pin
 // 415-417, Cloth::new cloth.rs:20-113), plus the device-layout builders:
 // CSR incidence lists for the general gather and the owned-strut parameter
-// planes for the grid stencil kernel.
+// records for the grid stencil kernel.
 #pragma once
 
 #include <stdint.h>
@@ -110,7 +110,7 @@ bool build_compact(const MeshTopo& m, const CsrTopo& t, CompactTopo& out);
 // exactly its binding struts after the triangle struts, and the strut ids
 // around every vertex ascend in the order the grid kernel sums them.
 bool grid_layout_ok(const MeshTopo& m);
-// Owned-strut constants, 4 float4 planes of n entries (see grid_order.h).
-void build_grid_params(const MeshTopo& m, std::vector<float>& planes /*16*n*/);
+// Strut constants of a grid (grid_order.h: param_rec).
+void build_grid_params(const MeshTopo& m, std::vector<float>& params);
 
 }  // namespace fgb

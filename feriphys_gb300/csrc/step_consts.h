@@ -28,8 +28,24 @@ struct ObsGrid3 {
   int always_base, n_always;  // faces tested for every query (in `always`)
 };
 
+// What the tiled kernel tests a move against before it starts the search: per
+// obstacle that has faces the box around their regions and the cells in it (as
+// in ObsGrid3), so that a move in an empty cell ends there.  The last entry
+// stands for all obstacles that do not get their own (the union of their
+// boxes), without cells (n[0] = 0: the search decides); so does, unbounded, an
+// obstacle with faces tested for every query.
+constexpr int kObsBoxes = 4;
+struct ObsBox {
+  float lo[3], hi[3];
+  float cell[3], inv[3], slack;
+  int n[3];
+  int off_base;
+};
+
 struct ObsAccel {
   int enabled;
+  int n_boxes;
+  ObsBox box[kObsBoxes];
   int n_grids;
   const ObsGrid3* grids;
   const int* cell_off;

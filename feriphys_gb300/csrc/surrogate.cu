@@ -1019,20 +1019,8 @@ __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ clot
   if (v < n) {
     const int r = v / C, col = v % C;
     const float4 p = P[v], vel = Vl[v];
-    // the vertex's owned-strut constants: one row of each of the four planes
-    float prm[16];
-    {
-      const float4 q0 = c.planes[v], q1 = c.planes[size_t(n) + v], q2 = c.planes[2 * size_t(n) + v],
-                   q3 = c.planes[3 * size_t(n) + v];
-      const float4 q[4] = {q0, q1, q2, q3};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        prm[4 * j] = q[j].x;
-        prm[4 * j + 1] = q[j].y;
-        prm[4 * j + 2] = q[j].z;
-        prm[4 * j + 3] = q[j].w;
-      }
-    }
+    const float* __restrict__ prm = c.params + grid::param_rec(r, col, C);
+    const int pc = col % 16, lane = (col / 16) % 2;
     E = 0.5f * p.w * ((vel.x * vel.x + vel.y * vel.y) + vel.z * vel.z) - ((gf.x * p.x + gf.y * p.y) + gf.z * p.z);
 #pragma unroll
     for (int kind = 0; kind < 5; ++kind) {
@@ -1048,8 +1036,8 @@ __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ clot
       const float4 pa = a == v ? p : P[a], pb = P[b];
       const float dx = pb.x - pa.x, dy = pb.y - pa.y, dz = pb.z - pa.z;
       const float d = sqrtf((dx * dx + dy * dy) + dz * dz);
-      const float k = prm[grid::param_index(kind, 0)];
-      const float L = prm[grid::param_index(kind, 2)];
+      const float k = prm[64 * kind + 4 * pc + lane];
+      const float L = prm[320 + 32 * kind + 2 * pc + lane];
       const float e = d - L;
       E += 0.5f * k * (e * e);
       S = fmaxf(S, fabsf(e / L));

@@ -73,7 +73,7 @@ struct Norm {
 struct SurCloth {
   float4* pos[2];
   float4* vel[2];
-  const float4* planes;  // owned-strut constants (grid_order.h), for the checks
+  const float* params;   // strut constants (grid_order.h: param_rec), for the checks
   const float4* rest;    // positions the mesh was built from (x, y, z, 0)
   unsigned* flags;       // bit 0: a vertex went non-finite
   int rows, cols;

@@ -1,0 +1,157 @@
+"""The tiled kernel's packed arithmetic and its rare branches on the GPU.
+
+* pair.cuh: the root of two lanes is the IEEE square root, and the reciprocal
+  of such a root the IEEE reciprocal, for every float in the stated range and,
+  for the form that also takes zeros, for zero.
+* The tiled kernel gives the bits of the general gather where its terms leave
+  the fast range (coincident points at the cloth's edges, no wind on a flat
+  cloth, extreme and non-finite coordinates), with carried forces, with the
+  reference's RK4, and with more obstacles than have a box of their own.
+"""
+import ctypes as C
+import os
+import subprocess
+import tempfile
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+KERNEL = r"""
+#include "pair.cuh"
+using namespace fgb;
+__global__ void roots(unsigned long long* bad) {
+  unsigned long long b[3] = {0, 0, 0};
+  for (unsigned long long i = kRootLo + blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+       i <= kRootLo + (unsigned long long)kRootSpan; i += (unsigned long long)gridDim.x * blockDim.x) {
+    const float x = __uint_as_float(unsigned(i)), x2 = __uint_as_float(unsigned(i) ^ 1u);
+    const float r = __fsqrt_rn(x), r2 = __fsqrt_rn(x2);
+    const float2 s = upk(root_fast2(pk(x, x2)));
+    if (s.x != r || s.y != r2) ++b[0];
+    const float2 q = upk(rcp_root_fast2(pk(r, r2)));
+    if (q.x != __fdiv_rn(1.0f, r) || q.y != __fdiv_rn(1.0f, r2)) ++b[1];
+    uint32_t far = 0;
+    const float2 z = upk(root_or_zero<true>(pk(x, 0.0f), far));
+    if (z.x != r || __float_as_uint(z.y) != 0u || far > kRootSpan) ++b[2];
+  }
+  for (int j = 0; j < 3; ++j)
+    if (b[j]) atomicAdd(bad + j, b[j]);
+}
+extern "C" int run_roots(unsigned long long* out) {
+  unsigned long long* d;
+  if (cudaMalloc(&d, 24) != cudaSuccess) return -1;
+  cudaMemset(d, 0, 24);
+  roots<<<4096, 256>>>(d);
+  if (cudaMemcpy(out, d, 24, cudaMemcpyDeviceToHost) != cudaSuccess) return -2;
+  cudaFree(d);
+  return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def fgb():
+    import feriphys_gb300
+
+    feriphys_gb300._lib()
+    return feriphys_gb300
+
+
+def test_roots_exact():
+    d = tempfile.mkdtemp(prefix="fgb_pair_")
+    src, lib = os.path.join(d, "pair.cu"), os.path.join(d, "libpair.so")
+    open(src, "w").write(KERNEL)
+    subprocess.check_call(["nvcc", "-O3", "-std=c++17", "-gencode", "arch=compute_103a,code=sm_103a", "-fmad=false",
+                           "-Xcompiler", "-fPIC", "-shared", "-I", os.path.join(ROOT, "feriphys_gb300", "csrc"),
+                           "-o", lib, src])
+    l = C.CDLL(lib)
+    out = (C.c_ulonglong * 3)()
+    assert l.run_roots(out) == 0
+    assert list(out) == [0, 0, 0]
+
+
+def _run(fgb, W, path, rows, cols, edit, steps=3, rk4=False, wind=(2.0, 0.0, 1.0), obstacles=None, force=False):
+    s = 1.0 / 31
+    lt, ls, lb = s, s * 2 ** 0.5, 2 * s
+    args = (rows, cols, s, (0.0, 0.0, 0.0), 0.01, 500 * lt, 0.5 * lt, 250 * ls, 0.5 * ls, 50 * lb, 0.5 * lb)
+    mesh = fgb.Cloth.new(*args, [0]).mesh
+    mesh.set_path(path)
+    obs = [W.plane(-0.3)] if obstacles is None else obstacles
+    sim = fgb.Simulation.new([mesh], [fgb.CollidableMesh.new(*o) for o in obs])
+    cfg = W.cloth_config(1.0 / 6000.0, 1 if rk4 else 0)
+    cfg["wind"] = wind
+    sim.set_config(fgb.Config.make(**cfg))
+    p = mesh.get_points()
+    edit(p.reshape(rows, cols, 10))
+    if force:
+        p[:, 7:10] = np.random.default_rng(1).normal(0, 0.01, (rows * cols, 3))
+    sim.step(0)
+    mesh.set_points(p)  # on the device already: the forces are carried into the first step
+    sim.step(steps)
+    return np.ascontiguousarray(mesh.get_points())
+
+
+def _same(a, b):
+    """Bit for bit, every NaN equal to every other."""
+    nan = np.isnan(a) & np.isnan(b)
+    return ((a.view(np.uint32) == b.view(np.uint32)) | nan).all()
+
+
+def _jitter(q):
+    q[..., 1:7] += np.random.default_rng(q.size).normal(0, 2e-3, q[..., 1:7].shape).astype(np.float32)
+
+
+def _coincident(q):
+    q[-1, :, 1:4] = q[-2, :, 1:4]  # the last two rows, which own no binding struts, on top of each other
+    q[:, -1, 1:4] = q[:, max(q.shape[1] - 3, 0), 1:4]
+    q[0, 0, 1:4] = q[0, 1, 1:4]
+
+
+def _far_away(q):
+    q[..., 1:4] *= np.float32(2.0 ** 62)
+
+
+def _huge_row(q):
+    _jitter(q)
+    q[q.shape[0] // 2, :, 1:4] *= np.float32(1e30)
+
+
+def _broken(q):
+    _jitter(q)
+    q[1, 1, 1] = np.nan
+    q[-1, -1, 2] = np.inf
+    q[0, -1, 4] = np.inf
+
+
+CASES = {"jitter": _jitter, "flat": lambda q: None, "coincident": _coincident, "far_away": _far_away,
+         "huge_row": _huge_row, "broken": _broken}
+
+
+@pytest.mark.parametrize("rows,cols", [(2, 2), (5, 16), (9, 33), (20, 50), (40, 170)])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_tiled_equals_general(fgb, case, rows, cols):
+    from feriphys_gb300 import workloads as W
+
+    for rk4, wind in ((False, (2.0, 0.0, 1.0)), (True, (0.0, 0.0, 0.0)), (False, (0.0, 0.0, 3.0))):
+        a, b = (_run(fgb, W, p, rows, cols, CASES[case], rk4=rk4, wind=wind) for p in (1, 2))
+        assert _same(a, b), (rk4, wind)
+
+
+@pytest.mark.parametrize("rows,cols", [(8, 32), (70, 95), (300, 200)])
+def test_carried_forces_and_many_obstacles(fgb, rows, cols):
+    """Sizes on both sides of the tile-height rule; five spheres through the cloth and a plane under it."""
+    from feriphys_gb300 import workloads as W
+
+    x, y = cols / 62.0, rows / 62.0
+    obs = [W.plane(-0.8 * y)] + [W.uv_sphere((a * x, b * y, 0.01), 0.2 * min(x, y), 12, 8)
+                                 for a, b in ((0, 0), (0.6, 0.5), (-0.6, 0.5), (0.6, -0.5), (-0.6, -0.5))]
+
+    def edit(q):
+        _jitter(q)
+        q[..., 6] += np.random.default_rng(3).normal(0, 20.0, q[..., 6].shape).astype(np.float32)
+
+    a, b = (_run(fgb, W, p, rows, cols, edit, steps=20, obstacles=obs, force=True) for p in (1, 2))
+    assert np.isfinite(a).all() and _same(a, b)
