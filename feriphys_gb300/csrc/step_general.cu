@@ -40,7 +40,7 @@ namespace fgb {
 
 namespace {
 
-// One strut term and one face term, added to F in the reference's order.
+// One strut term added to F, and one face term, in the reference's order.
 template <class T>
 __device__ __forceinline__ void add_strut(V3<T>& F, V3<T> P, V3<T> V, V3<T> Po, V3<T> Vo, int role, float k,
                                           float cd, float L) {
@@ -56,14 +56,12 @@ __device__ __forceinline__ void add_strut(V3<T>& F, V3<T> P, V3<T> V, V3<T> Po, 
   }
 }
 template <class T>
-__device__ __forceinline__ void add_face(V3<T>& F, int i0, int i1, int i2, int corner,
-                                         const Vec4<T>* __restrict__ pos, const Vec4<T>* __restrict__ vel,
-                                         V3<T> wind, const StepConsts& c) {
+__device__ __forceinline__ V3<T> face_term(int i0, int i1, int i2, int corner, const Vec4<T>* __restrict__ pos,
+                                           const Vec4<T>* __restrict__ vel, V3<T> wind, const StepConsts& c) {
   const V3<T> x0 = xyz<T>(pos[i0]), x1 = xyz<T>(pos[i1]), x2 = xyz<T>(pos[i2]);
   const V3<T> v0 = xyz<T>(vel[i0]), v1 = xyz<T>(vel[i1]), v2 = xyz<T>(vel[i2]);
   const V3<T> total = face_total_force<T>(x0, x1, x2, v0, v1, v2, wind, T(c.neg_drag), T(c.neg_lift));
-  const T w = face_corner_weight<T>(x0, x1, x2, corner);
-  F = F + w * total;
+  return face_corner_weight<T>(x0, x1, x2, corner) * total;
 }
 
 // A strut word of form 1 (32 bits) or 2 (16 bits; a role-0 word has no rank
@@ -83,12 +81,11 @@ __device__ __forceinline__ void strut_word(const GeneralTopo& t, int e, int& off
   }
 }
 
+// Strut terms of vertex v added to F in strut order.
 template <class T, int FORM>
-__device__ __forceinline__ V3<T> gather_forces(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* __restrict__ pos,
-                                               const Vec4<T>* __restrict__ vel, const GeneralTopo& t,
-                                               const StepConsts& c) {
+__device__ __forceinline__ V3<T> gather_struts(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* __restrict__ pos,
+                                               const Vec4<T>* __restrict__ vel, const GeneralTopo& t) {
   const int s_beg = t.strut_off[v], s_end = t.strut_off[v + 1];
-  const V3<T> wind{T(c.wind[0]), T(c.wind[1]), T(c.wind[2])};
   if constexpr (FORM != 0) {
     int own = t.own_off[v];  // owner position of v's next role-0 strut
     for (int e = s_beg; e < s_end; ++e) {
@@ -99,31 +96,45 @@ __device__ __forceinline__ V3<T> gather_forces(int v, V3<T> P, V3<T> V, V3<T> F,
       add_strut<T>(F, P, V, xyz<T>(pos[o]), xyz<T>(vel[o]), role, __ldg(t.sk + i), __ldg(t.sc + i),
                    __ldg(t.sl + i));
     }
-    const int f_beg = t.face_off[v], f_end = t.face_off[v + 1];
-    for (int e = f_beg; e < f_end; ++e) {
-      const uint32_t h = __ldg(t.face_word + e);
-      const int corner = int(h & 3u);
-      int o1, o2, rk, rl;
-      strut_word<FORM>(t, s_beg + int((h >> 2) & 127u), o1, rk, rl);
-      strut_word<FORM>(t, s_beg + int(h >> 9), o2, rk, rl);
-      const int u1 = v + o1, u2 = v + o2;
-      const int i0 = corner == 0 ? v : u1, i1 = corner == 0 ? u1 : (corner == 1 ? v : u2),
-                i2 = corner == 2 ? v : u2;
-      add_face<T>(F, i0, i1, i2, corner, pos, vel, wind, c);
-    }
   } else {
     for (int e = s_beg; e < s_end; ++e) {
       const int2 inc = t.strut_inc[e];
       const float4 kcl = t.strut_kcl[inc.y >> 1];
       add_strut<T>(F, P, V, xyz<T>(pos[inc.x]), xyz<T>(vel[inc.x]), inc.y & 1, kcl.x, kcl.y, kcl.z);
     }
-    const int f_beg = t.face_off[v], f_end = t.face_off[v + 1];
-    for (int e = f_beg; e < f_end; ++e) {
-      const int fc = t.face_inc[e];
-      const int4 fv = t.face_vtx[fc >> 2];
-      add_face<T>(F, fv.x, fv.y, fv.z, fc & 3, pos, vel, wind, c);
-    }
   }
+  return F;
+}
+
+// The share of v in its face incidence e (s_beg: v's first strut incidence).
+template <class T, int FORM>
+__device__ __forceinline__ V3<T> face_share(int v, int e, int s_beg, const Vec4<T>* __restrict__ pos,
+                                            const Vec4<T>* __restrict__ vel, const GeneralTopo& t, V3<T> wind,
+                                            const StepConsts& c) {
+  if constexpr (FORM != 0) {
+    const uint32_t h = __ldg(t.face_word + e);
+    const int corner = int(h & 3u);
+    int o1, o2, rk, rl;
+    strut_word<FORM>(t, s_beg + int((h >> 2) & 127u), o1, rk, rl);
+    strut_word<FORM>(t, s_beg + int(h >> 9), o2, rk, rl);
+    const int u1 = v + o1, u2 = v + o2;
+    const int i0 = corner == 0 ? v : u1, i1 = corner == 0 ? u1 : (corner == 1 ? v : u2), i2 = corner == 2 ? v : u2;
+    return face_term<T>(i0, i1, i2, corner, pos, vel, wind, c);
+  } else {
+    const int fc = t.face_inc[e];
+    const int4 fv = t.face_vtx[fc >> 2];
+    return face_term<T>(fv.x, fv.y, fv.z, fc & 3, pos, vel, wind, c);
+  }
+}
+
+template <class T, int FORM>
+__device__ __forceinline__ V3<T> gather_forces(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* __restrict__ pos,
+                                               const Vec4<T>* __restrict__ vel, const GeneralTopo& t,
+                                               const StepConsts& c) {
+  const V3<T> wind{T(c.wind[0]), T(c.wind[1]), T(c.wind[2])};
+  F = gather_struts<T, FORM>(v, P, V, F, pos, vel, t);
+  const int s_beg = t.strut_off[v], f_beg = t.face_off[v], f_end = t.face_off[v + 1];
+  for (int e = f_beg; e < f_end; ++e) F = F + face_share<T, FORM>(v, e, s_beg, pos, vel, t, wind, c);
   return F;
 }
 
@@ -134,13 +145,16 @@ __device__ __forceinline__ void flag_nonfinite(bool bad, unsigned* flags) {
 // Fused Simulation::step for one mesh (accumulate -> integrate -> collide ->
 // pin restore -> clear), one thread per vertex.  The f32 form asks for 4
 // blocks of 256 per SM (at most 64 registers: the gather is latency-bound, so
-// resident warps count); the FP64 rerun keeps the registers it needs.
+// resident warps count); the FP64 rerun, bound by the FP64 units (one warp
+// instruction takes one of them 64 cycles), takes single-warp blocks so that a
+// mesh reaches as many of them as it has warps (90 x 61 tube: 123 us a step
+// with blocks of 256, 64 with 32).
+template <class T> constexpr int kStepBlock = sizeof(T) == 4 ? 256 : 32;
 template <class T, int FORM>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_step_general(int n, const Vec4<T>* __restrict__ pos,
-                                                      const Vec4<T>* __restrict__ vel,
-                                                      const Vec4<T>* __restrict__ force_in,
-                                                      Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
-                                                      GeneralTopo t, StepConsts c) {
+__global__ void __launch_bounds__(kStepBlock<T>, sizeof(T) == 4 ? 4 : 1)
+    k_step_general(int n, const Vec4<T>* __restrict__ pos, const Vec4<T>* __restrict__ vel,
+                   const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
+                   GeneralTopo t, StepConsts c) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
   const Vec4<T> P4 = pos[v];
@@ -160,6 +174,85 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_step_general(in
     F = V3<T>{T(c.force0[0]), T(c.force0[1]), T(c.force0[2])};
   }
   F = gather_forces<T, FORM>(v, P, V, F, pos, vel, t, c);
+  V3<T> np, nv, nF;
+  integrate_point<T>(c.integration, T(c.dt), P, V, F, m, np, nv, nF);
+  collide_point<T>(static_cast<const ObsFace*>(c.obstacle_faces), c.n_obstacle_faces, P, V, F, m, np, nv, c);
+  pos_out[v] = make4<T>(np, m);
+  vel_out[v] = make4<T>(nv, V4.w);
+  flag_nonfinite(!(finite3(np) && finite3(nv)), c.flags);
+}
+
+// The same step with a vertex's terms spread over the warps of a block: 32
+// vertices a block, warp 0 sums their struts, the NF other warps compute their
+// face shares (warp 1 + j the faces j, j + NF, ...) into shared memory, and
+// warp 0 adds those in face order, integrates and collides.  The same terms in
+// the same order, so the same bits as k_step_general; a vertex's chain of
+// terms is what a step of a small or slow mesh waits for (see the launch).
+template <class T> struct SplitShape;
+template <> struct SplitShape<float> { static constexpr int NF = 3, PER = 2; };
+template <> struct SplitShape<double> { static constexpr int NF = 6, PER = 1; };
+
+template <class T, int FORM>
+__global__ void __launch_bounds__(32 * (SplitShape<T>::NF + 1))
+    k_step_split(int n, const Vec4<T>* __restrict__ pos, const Vec4<T>* __restrict__ vel,
+                 const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
+                 GeneralTopo t, StepConsts c) {
+  constexpr int NF = SplitShape<T>::NF, PER = SplitShape<T>::PER, SLOTS = NF * PER;
+  __shared__ T share[SLOTS][3][32];
+  __shared__ int s_rounds;
+  const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
+  const int v = blockIdx.x * 32 + lane;
+  const bool vertex = v < n;
+  const Vec4<T> V4 = vertex ? vel[v] : make4<T>(V3<T>{T(0), T(0), T(0)}, T(1));
+  const bool free = vertex && V4.w == T(0);  // pinned: update_points restores the old point
+  const int f_beg = free ? t.face_off[v] : 0, f_end = free ? t.face_off[v + 1] : 0;
+  if (role == 0) {
+    const int most = __reduce_max_sync(0xffffffffu, f_end - f_beg);
+    if (lane == 0) s_rounds = (most + SLOTS - 1) / SLOTS;
+  }
+  Vec4<T> P4 = V4;
+  V3<T> F{T(0), T(0), T(0)};
+  if (role == 0) {
+    if (vertex) P4 = pos[v];
+    if (free) {
+      const V3<T> g{T(c.force0[0]), T(c.force0[1]), T(c.force0[2])};
+      F = force_in ? xyz<T>(force_in[v]) + g : g;
+      F = gather_struts<T, FORM>(v, xyz<T>(P4), xyz<T>(V4), F, pos, vel, t);
+    }
+  }
+  auto shares = [&](int round) {
+    const V3<T> wind{T(c.wind[0]), T(c.wind[1]), T(c.wind[2])};
+    const int s_beg = free ? t.strut_off[v] : 0;
+#pragma unroll 1
+    for (int j = role - 1; j < SLOTS; j += NF) {
+      const int e = f_beg + round * SLOTS + j;
+      if (e >= f_end) break;
+      const V3<T> w = face_share<T, FORM>(v, e, s_beg, pos, vel, t, wind, c);
+      share[j][0][lane] = w.x;
+      share[j][1][lane] = w.y;
+      share[j][2][lane] = w.z;
+    }
+  };
+  if (role > 0) shares(0);
+  __syncthreads();
+  for (int round = 0; round < s_rounds; ++round) {
+    if (round > 0) {
+      if (role > 0) shares(round);
+      __syncthreads();
+    }
+    if (role == 0)
+      for (int j = 0; j < SLOTS && f_beg + round * SLOTS + j < f_end; ++j)
+        F = F + V3<T>{share[j][0][lane], share[j][1][lane], share[j][2][lane]};
+    if (round + 1 < s_rounds) __syncthreads();
+  }
+  if (role != 0 || !vertex) return;
+  if (!free) {
+    pos_out[v] = P4;
+    vel_out[v] = V4;
+    return;
+  }
+  const V3<T> P = xyz<T>(P4), V = xyz<T>(V4);
+  const T m = P4.w;
   V3<T> np, nv, nF;
   integrate_point<T>(c.integration, T(c.dt), P, V, F, m, np, nv, nF);
   collide_point<T>(static_cast<const ObsFace*>(c.obstacle_faces), c.n_obstacle_faces, P, V, F, m, np, nv, c);
@@ -233,10 +326,23 @@ template <class T>
 cudaError_t launch_step_general(int n, const void* pos, const void* vel, const void* force_in, void* pos_out,
                                 void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  auto k = t.form == 2 ? k_step_general<T, 2> : (t.form == 1 ? k_step_general<T, 1> : k_step_general<T, 0>);
-  k<<<blocks_for(n, 256), 256, 0, s>>>(n, static_cast<const Vec4<T>*>(pos), static_cast<const Vec4<T>*>(vel),
-                                       static_cast<const Vec4<T>*>(force_in), static_cast<Vec4<T>*>(pos_out),
-                                       static_cast<Vec4<T>*>(vel_out), t, c);
+  const auto run = [&](auto kernel, int blocks, int threads) {
+    kernel<<<blocks, threads, 0, s>>>(n, static_cast<const Vec4<T>*>(pos), static_cast<const Vec4<T>*>(vel),
+                                      static_cast<const Vec4<T>*>(force_in), static_cast<Vec4<T>*>(pos_out),
+                                      static_cast<Vec4<T>*>(vel_out), t, c);
+  };
+  // Up to this many vertices a step takes as long as one vertex's chain of
+  // terms, which the split kernel shortens; beyond, the SMs are full and its
+  // shared-memory exchange only costs (tubes, us a step, one thread per vertex
+  // against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3, 360 x 280 14.4
+  // -> 18.6; FP64 12 x 10 64 -> 29, 90 x 61 64 -> 39, 300 x 200 207 -> 220).
+  constexpr int kSplitMost = 32768;
+  if (n <= kSplitMost)
+    run(t.form == 2 ? k_step_split<T, 2> : (t.form == 1 ? k_step_split<T, 1> : k_step_split<T, 0>),
+        blocks_for(n, 32), 32 * (SplitShape<T>::NF + 1));
+  else
+    run(t.form == 2 ? k_step_general<T, 2> : (t.form == 1 ? k_step_general<T, 1> : k_step_general<T, 0>),
+        blocks_for(n, kStepBlock<T>), kStepBlock<T>);
   return cudaGetLastError();
 }
 

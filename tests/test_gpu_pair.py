@@ -155,3 +155,35 @@ def test_carried_forces_and_many_obstacles(fgb, rows, cols):
 
     a, b = (_run(fgb, W, p, rows, cols, edit, steps=20, obstacles=obs, force=True) for p in (1, 2))
     assert np.isfinite(a).all() and _same(a, b)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("valence", [3, 6, 7, 13, 40])
+def test_split_step_any_valence(fgb, orc, bits, valence):
+    """A fan around one vertex of the given valence beside a strip, in a mesh
+    small enough for the split general step (several rounds of face shares for
+    the hub, none for a loose point), against the oracle."""
+    rng = np.random.default_rng(valence)
+    a = np.linspace(0, 2 * np.pi, valence, endpoint=False)
+    ring = np.stack([np.cos(a), np.sin(a), 0.1 * np.cos(3 * a)], 1)
+    extra = rng.normal(0, 1, (9, 3)) + 3.0
+    pos = np.concatenate([[[0, 0, 0.2]], ring, extra]).astype(np.float32)
+    idx = [x for k in range(valence) for x in (0, 1 + k, 1 + (k + 1) % valence)]
+    b = 1 + valence
+    idx += [x for k in range(6) for x in (b + k, b + k + 1, b + k + 2)]  # leaves the last point loose
+    m = fgb.SpringyMesh.new(pos, idx, 0.01 * len(pos), 5.0, 0.01)
+    m.add_pins([b])
+    m.set_precision(bits)
+    cfg = dict(dt=1.0 / 6000.0, gravity=(0.0, -0.1, 0.0), wind=(2.0, 0.5, 1.0))
+    sim = fgb.Simulation.new([m], [])
+    sim.set_config(fgb.Config.make(lift_coefficient=0.3, drag_coefficient=0.6, coefficient_of_restitution=0.3,
+                                   coefficient_of_friction=0.2, **cfg))
+    om = orc.SpringyMesh.new(pos, np.array(idx, np.uint32), 0.01 * len(pos), 5.0, 0.01)
+    om.add_pins(np.array([b], np.uint32))
+    osim = orc.Simulation([om], [])
+    osim.set_config(orc.Config.make(0, cfg["dt"], cfg["gravity"], cfg["wind"], 0.3, 0.6, 0.3, 0.2))
+    for _ in range(5):
+        sim.step(1)
+        osim.step(1)
+    g, o = m.get_points()[:, 1:7].astype(np.float64), om.get_points()[:, 1:7].astype(np.float64)
+    assert np.abs(g - o).max() / np.abs(o).max() <= 1e-6  # five steps of f32 rounding; the terms are O(1) of the state
