@@ -5,9 +5,10 @@
 // Vector3::angle(a, b) = atan2(|a x b|, a . b).  The library is compiled with
 // -fmad=false so no a*b+c is fused, and '/' and sqrt are the IEEE-rounded
 // operations; with the same operation order the results are bit-identical to
-// the reference's f32 arithmetic except in the faces' corner angles: the
-// atan2 is the library's own (angle.cuh), and the three corners share one
-// cross-product magnitude (physics.cuh: face_corner_weight).
+// the reference's f32 arithmetic except in the face terms: sums of products
+// are fused, drag and lift are one factor of the relative velocity, the atan2
+// is the library's own (angle.cuh), and the three corners share one
+// cross-product magnitude (physics.cuh: face_total_force, face_corner_weight).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -51,6 +52,20 @@ template <class T> __device__ __forceinline__ T dot(V3<T> a, V3<T> b) { return a
 template <class T> __device__ __forceinline__ V3<T> cross(V3<T> a, V3<T> b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
+// The same with the second product fused (one rounding less each): the face
+// terms of both precisions, and everything of the FP64 rerun -- its error is
+// far below what it is used to state, and the FP64 units bound it (300 x 200
+// tube 207 -> 144 us a step).
+__device__ __forceinline__ float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fused(double a, double b, double c) { return fma(a, b, c); }
+template <class T> __device__ __forceinline__ T fdot(V3<T> a, V3<T> b) {
+  return fused(a.z, b.z, fused(a.y, b.y, a.x * b.x));
+}
+template <class T> __device__ __forceinline__ V3<T> fcross(V3<T> a, V3<T> b) {
+  return {fused(a.y, b.z, -(a.z * b.y)), fused(a.z, b.x, -(a.x * b.z)), fused(a.x, b.y, -(a.y * b.x))};
+}
+__device__ __forceinline__ double dot(V3<double> a, V3<double> b) { return fdot(a, b); }
+__device__ __forceinline__ V3<double> cross(V3<double> a, V3<double> b) { return fcross(a, b); }
 __device__ __forceinline__ float sq_root(float v) { return sqrtf(v); }
 __device__ __forceinline__ double sq_root(double v) { return sqrt(v); }
 // atan2(y, x) for y >= 0 (the angle between two vectors: cgmath's

@@ -26,53 +26,44 @@ __device__ __forceinline__ void strut_forces(V3<T> p0, V3<T> p1, V3<T> v0, V3<T>
   df = (c * dot(v1 - v0, u)) * u;
 }
 
-// drag + lift of one face (springy_mesh.rs:634-646).  The f32 step takes
-// the mean velocity as the sum times RN(1/3) (the reference divides by 3: at
-// most an ulp apart, in the face terms only); the FP64 rerun divides.
+// drag + lift of one face (springy_mesh.rs:634-646): with the face's area A,
+// unit normal n and e = A |n . rv| the reference's
+// -Cd e rv - Cl e |n x rv| rv as one factor times rv, the mean velocity as the
+// sum times RN(1/3) where the reference divides by 3, and sums of products
+// fused.  Fewer roundings than the reference's sequence, in the face terms only.
 template <class T>
 __device__ __forceinline__ V3<T> face_total_force(V3<T> x0, V3<T> x1, V3<T> x2, V3<T> v0, V3<T> v1, V3<T> v2,
                                                   V3<T> wind, T neg_cd, T neg_cl) {
-  V3<T> avg;
-  if constexpr (sizeof(T) == 8) avg = ((v0 + v1) + v2) / T(3);
-  else avg = ((v0 + v1) + v2) * kRcp3;
-  const V3<T> rv = avg - wind;
-  const V3<T> cr = cross(x1 - x0, x2 - x0);
-  const T area = magnitude(cr) / T(2);
-  const V3<T> n = normalize(cr);
-  const T eff = area * abs_val(dot(n, rv));
-  const V3<T> drag = (neg_cd * eff) * rv;
-  const V3<T> lift = (neg_cl * eff) * (rv * magnitude(cross(n, rv)));
-  return drag + lift;
+  const V3<T> sum = (v0 + v1) + v2;
+  const T r3 = sizeof(T) == 8 ? T(1.0 / 3.0) : T(kRcp3);
+  const V3<T> rv{fused(sum.x, r3, -wind.x), fused(sum.y, r3, -wind.y), fused(sum.z, r3, -wind.z)};
+  const V3<T> cr = fcross(x1 - x0, x2 - x0);
+  const T mag = sq_root(fdot(cr, cr));
+  const V3<T> n = cr * inv_magnitude(mag);
+  const T eff = (mag * T(0.5)) * abs_val(fdot(n, rv));
+  const V3<T> nr = fcross(n, rv);
+  return (eff * fused(neg_cl, sq_root(fdot(nr, nr)), neg_cd)) * rv;
 }
 
 // Vertex angle of corner k over PI (springy_mesh.rs:134-172, 647-649).  The
 // reference takes each corner's angle as atan2(|a x b|, a . b) of that
-// corner's two edges; the FP64 rerun (T = double) does exactly that.  The f32
-// step saves work the reference repeats: |a x b| is twice the face's area at
-// every corner, so corners 0 and 1 take the one magnitude
-// |(x1 - x0) x (x2 - x0)| the drag already needs, with their own dot products
-// in the reference's order; the angles sum to pi, so corner 2's share is
-// (1 - w0) - w1; and a share is the angle times RN(1/pi) instead of over pi.
-// Each differs from the reference's per-corner computation by rounding only
-// (about 1e-7 of the face's force), like the angle's own last bits.
+// corner's two edges.  |a x b| is twice the face's area at every corner, so
+// all take the one magnitude |(x1 - x0) x (x2 - x0)| the drag already needs,
+// with their own dot products; a share is the angle times the reciprocal of the
+// reference's f32 pi instead of over it; and in f32 the angles summing to pi makes corner 2's share
+// (1 - w0) - w1.  Each differs from the reference's per-corner computation by
+// rounding only (in f32 about 1e-7 of the face's force).
 template <class T>
 __device__ __forceinline__ T corner_share(V3<T> x0, V3<T> x1, V3<T> x2, T y, int k) {
-  const T x = k == 0 ? dot(x2 - x0, x1 - x0) : dot(x0 - x1, x2 - x1);
-  return angle_of(y, x) * kRcpPi;
+  const T x = k == 0 ? fdot(x2 - x0, x1 - x0) : (k == 1 ? fdot(x0 - x1, x2 - x1) : fdot(x1 - x2, x0 - x2));
+  return angle_of(y, x) * (sizeof(T) == 8 ? T(1.0 / double(kPiF32)) : T(kRcpPi));
 }
 template <class T>
 __device__ __forceinline__ T face_corner_weight(V3<T> x0, V3<T> x1, V3<T> x2, int k) {
-  if constexpr (sizeof(T) == 8) {  // the reference's form
-    V3<T> a, b;
-    if (k == 0) { a = x2 - x0; b = x1 - x0; }
-    else if (k == 1) { a = x0 - x1; b = x2 - x1; }
-    else { a = x1 - x2; b = x0 - x2; }
-    return angle_of(magnitude(cross(a, b)), dot(a, b)) / T(kPiF32);
-  } else {
-    const T y = magnitude(cross(x1 - x0, x2 - x0));
-    if (k < 2) return corner_share(x0, x1, x2, y, k);
-    return (T(1) - corner_share(x0, x1, x2, y, 0)) - corner_share(x0, x1, x2, y, 1);
-  }
+  const V3<T> cr = fcross(x1 - x0, x2 - x0);
+  const T y = sq_root(fdot(cr, cr));
+  if (sizeof(T) == 8 || k < 2) return corner_share(x0, x1, x2, y, k);
+  return (T(1) - corner_share(x0, x1, x2, y, 0)) - corner_share(x0, x1, x2, y, 1);
 }
 
 // F / m componentwise, exactly as IEEE division; the f32 form shares one

@@ -335,7 +335,8 @@ cudaError_t launch_step_general(int n, const void* pos, const void* vel, const v
   // terms, which the split kernel shortens; beyond, the SMs are full and its
   // shared-memory exchange only costs (tubes, us a step, one thread per vertex
   // against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3, 360 x 280 14.4
-  // -> 18.6; FP64 12 x 10 64 -> 29, 90 x 61 64 -> 39, 300 x 200 207 -> 220).
+  // -> 18.6; FP64, before its terms were fused, 12 x 10 64 -> 29, 90 x 61 64
+  // -> 39, 300 x 200 207 -> 220).
   constexpr int kSplitMost = 32768;
   if (n <= kSplitMost)
     run(t.form == 2 ? k_step_split<T, 2> : (t.form == 1 ? k_step_split<T, 1> : k_step_split<T, 0>),
