@@ -52,6 +52,7 @@ template <class T> __device__ __forceinline__ T dot(V3<T> a, V3<T> b) { return a
 template <class T> __device__ __forceinline__ V3<T> cross(V3<T> a, V3<T> b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
+#if defined(__CUDACC__)
 // The same with the second product fused (one rounding less each): the face
 // terms of both precisions, and everything of the FP64 rerun -- its error is
 // far below what it is used to state, and the FP64 units bound it (300 x 200
@@ -66,6 +67,7 @@ template <class T> __device__ __forceinline__ V3<T> fcross(V3<T> a, V3<T> b) {
 }
 __device__ __forceinline__ double dot(V3<double> a, V3<double> b) { return fdot(a, b); }
 __device__ __forceinline__ V3<double> cross(V3<double> a, V3<double> b) { return fcross(a, b); }
+#endif
 __device__ __forceinline__ float sq_root(float v) { return sqrtf(v); }
 __device__ __forceinline__ double sq_root(double v) { return sqrt(v); }
 // atan2(y, x) for y >= 0 (the angle between two vectors: cgmath's
