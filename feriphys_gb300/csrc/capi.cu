@@ -367,15 +367,15 @@ int step_mesh(fgb_mesh* m, const fgb::StepConsts& c) {
     FGB_CUDA(fgb::launch_step_grid(g, static_cast<const float4*>(m->pos[m->cur]),
                                    static_cast<const float4*>(m->vel[m->cur]), static_cast<const float4*>(F),
                                    static_cast<float4*>(m->pos[nxt]), static_cast<float4*>(m->vel[nxt]), c,
-                                   m->stream));
+                                   m->stream, true));
   } else {
     const fgb::GeneralTopo t = general_topo(m);
     if (m->precision == 64)
       FGB_CUDA(fgb::launch_step_general<double>(n, m->pos[m->cur], m->vel[m->cur], F, m->pos[nxt], m->vel[nxt], t,
-                                                c, m->stream));
+                                                c, m->stream, true));
     else
       FGB_CUDA(fgb::launch_step_general<float>(n, m->pos[m->cur], m->vel[m->cur], F, m->pos[nxt], m->vel[nxt], t,
-                                               c, m->stream));
+                                               c, m->stream, true));
   }
   m->cur = nxt;
   m->has_force = false;  // clear_forces
@@ -478,7 +478,7 @@ int prepare_batch(fgb_sim* s) {
 int batch_launch(fgb_sim* s, int parity) {
   FGB_CUDA(fgb::launch_step_batched(s->d_desc, s->d_work, s->n_work, parity,
                                     make_consts(s->cfg, s->d_faces, s->n_faces, nullptr, &s->accel), batch_stream(s),
-                                    nullptr, s->tile_h));
+                                    true, nullptr, s->tile_h));
   return FGB_OK;
 }
 
@@ -1484,7 +1484,7 @@ extern "C" int fgb_sim_step_static(fgb_sim* s, uint64_t n_steps, void* stream) {
   s->accel.enabled = (s->broadphase && s->d_accel) ? 1 : 0;
   for (uint64_t k = 0; k < n_steps; ++k) {
     FGB_CUDA(fgb::launch_step_batched(d_desc, d_work, int(n_work), int(k & 1),
-                                      make_consts(s->cfg, s->d_faces, s->n_faces, nullptr, &s->accel), st));
+                                      make_consts(s->cfg, s->d_faces, s->n_faces, nullptr, &s->accel), st, true));
     if (k == 0 && n_steps > 1) {  // carried forces apply to the first step only
       bool forces = false;
       for (const fgb::ClothDesc& d : desc) forces = forces || d.force_in;

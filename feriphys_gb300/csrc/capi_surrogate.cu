@@ -373,7 +373,7 @@ int fine_fallback(fgb_surrogate* g, fgb_sim* s, const std::vector<int>& failing,
       for (uint32_t j = 0; j < ratio; ++j, a ^= 1)
         FGB_CUDA(fgb::launch_step_grid(gt, static_cast<const float4*>(m->pos[a]), static_cast<const float4*>(m->vel[a]),
                                        nullptr, static_cast<float4*>(m->pos[a ^ 1]), static_cast<float4*>(m->vel[a ^ 1]),
-                                       mc, st));
+                                       mc, st, true));
       if (a != (par ^ 1)) {
         const size_t bytes = size_t(m->topo.n) * sizeof(float4);
         FGB_CUDA(cudaMemcpyAsync(m->pos[par ^ 1], m->pos[a], bytes, cudaMemcpyDeviceToDevice, st));
@@ -407,7 +407,7 @@ int fine_fallback(fgb_surrogate* g, fgb_sim* s, const std::vector<int>& failing,
     from = par ^ 1;
   }
   for (uint32_t j = 0; j < ratio && n_fw > 0; ++j)
-    FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, n_fw, from ^ int(j & 1u), fc, st, nullptr, s->tile_h));
+    FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, n_fw, from ^ int(j & 1u), fc, st, true, nullptr, s->tile_h));
   FGB_CUDA(cudaStreamSynchronize(st));  // the host table must outlive its upload
   return FGB_OK;
 }
@@ -439,7 +439,7 @@ int capture_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, c
     for (uint32_t j = 0; j < ro.ratio; ++j, a ^= 1)
       FGB_CUDA(fgb::launch_step_grid(gt, static_cast<const float4*>(m->pos[a]), static_cast<const float4*>(m->vel[a]),
                                      nullptr, static_cast<float4*>(m->pos[a ^ 1]), static_cast<float4*>(m->vel[a ^ 1]),
-                                     mc, bs));
+                                     mc, bs, false));
     if (a != (par ^ 1)) {
       const size_t bytes = size_t(m->topo.n) * sizeof(float4);
       FGB_CUDA(cudaMemcpyAsync(m->pos[par ^ 1], m->pos[a], bytes, cudaMemcpyDeviceToDevice, bs));
@@ -460,7 +460,7 @@ int capture_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, c
     }
     for (uint32_t j = 0; j < ro.ratio; ++j)
       FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, s->n_work, from ^ int(j & 1u), ro.fine, bs,
-                                        g->d_counts + 1, s->tile_h));
+                                        false, g->d_counts + 1, s->tile_h));
   }
   FGB_CUDA(S::launch_check(g->d_cloths, g->d_tiles, ro.n_tiles, ro.n_cloths, par ^ 1, ro.gforce, g->d_tile_chk,
                            g->d_cloth_chk, bs));

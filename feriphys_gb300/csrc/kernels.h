@@ -39,7 +39,8 @@ struct GridTopo {
 
 template <class T>
 cudaError_t launch_step_general(int n, const void* pos, const void* vel, const void* force_in, void* pos_out,
-                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s);
+                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s,
+                                bool chained);
 template <class T>
 cudaError_t launch_accumulate(int n, const void* pos, const void* vel, void* force, const GeneralTopo& t,
                               const StepConsts& c, cudaStream_t s);
@@ -52,8 +53,10 @@ cudaError_t launch_update(int n, void* pos, void* vel, void* force, const void* 
 template <class T>
 cudaError_t launch_zero4(int n, void* a, cudaStream_t s);
 
+// chained: the launch may overlap the end of the one before it in the stream
+// (chain_launch.cuh); false in the body of a conditional graph node.
 cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4* vel, const float4* force_in,
-                             float4* pos_out, float4* vel_out, const StepConsts& c, cudaStream_t s);
+                             float4* pos_out, float4* vel_out, const StepConsts& c, cudaStream_t s, bool chained);
 
 // One cloth of a batch (Cloth::new topology); buffers [parity] are read and
 // [parity ^ 1] written by a step.
@@ -86,7 +89,7 @@ int grid_tiles(int rows, int cols, int th, int* out3 /* may be null */);
 // (n_work is then its upper bound, which sizes the grid).
 // th: the tile height the work list was made for.
 cudaError_t launch_step_batched(const ClothDesc* cloths, const int4* work, int n_work, int parity,
-                                const StepConsts& c, cudaStream_t s, const int* n_work_dev = nullptr,
+                                const StepConsts& c, cudaStream_t s, bool chained, const int* n_work_dev = nullptr,
                                 int th = kDefaultTileH);
 // Sets the launch attributes of the tiled and batched step kernels (done by
 // their launchers on first use; call it before a stream capture).

@@ -33,6 +33,7 @@
 // plus 12 / 2 per strut incidence and 2 per face incidence, instead of
 // 8 + 16 and 4 + 16.  The terms and their order are the same, so are the
 // bits.
+#include "chain_launch.cuh"
 #include "kernels.h"
 #include "physics.cuh"
 
@@ -155,6 +156,8 @@ __global__ void __launch_bounds__(kStepBlock<T>, sizeof(T) == 4 ? 4 : 1)
     k_step_general(int n, const Vec4<T>* __restrict__ pos, const Vec4<T>* __restrict__ vel,
                    const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
                    GeneralTopo t, StepConsts c) {
+  chain_wait();
+  chain_next();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
   const Vec4<T> P4 = pos[v];
@@ -203,6 +206,8 @@ __global__ void __launch_bounds__(32 * (SplitShape<T>::NF + 1))
   const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
   const int v = blockIdx.x * 32 + lane;
   const bool vertex = v < n;
+  chain_wait();
+  chain_next();
   const Vec4<T> V4 = vertex ? vel[v] : make4<T>(V3<T>{T(0), T(0), T(0)}, T(1));
   const bool free = vertex && V4.w == T(0);  // pinned: update_points restores the old point
   const int f_beg = free ? t.face_off[v] : 0, f_end = free ? t.face_off[v + 1] : 0;
@@ -324,12 +329,13 @@ inline int blocks_for(int n, int bs) { return (n + bs - 1) / bs; }
 
 template <class T>
 cudaError_t launch_step_general(int n, const void* pos, const void* vel, const void* force_in, void* pos_out,
-                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s) {
+                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s,
+                                bool chained) {
   if (n <= 0) return cudaSuccess;
   const auto run = [&](auto kernel, int blocks, int threads) {
-    kernel<<<blocks, threads, 0, s>>>(n, static_cast<const Vec4<T>*>(pos), static_cast<const Vec4<T>*>(vel),
-                                      static_cast<const Vec4<T>*>(force_in), static_cast<Vec4<T>*>(pos_out),
-                                      static_cast<Vec4<T>*>(vel_out), t, c);
+    chain_launch(kernel, blocks, threads, 0, s, chained, n, static_cast<const Vec4<T>*>(pos),
+                 static_cast<const Vec4<T>*>(vel), static_cast<const Vec4<T>*>(force_in),
+                 static_cast<Vec4<T>*>(pos_out), static_cast<Vec4<T>*>(vel_out), t, c);
   };
   // Up to this many vertices a step takes as long as one vertex's chain of
   // terms, which the split kernel shortens; beyond, the SMs are full and its
@@ -388,7 +394,7 @@ cudaError_t launch_zero4(int n, void* a, cudaStream_t s) {
 
 #define FGB_INSTANTIATE(T)                                                                                        \
   template cudaError_t launch_step_general<T>(int, const void*, const void*, const void*, void*, void*,          \
-                                              const GeneralTopo&, const StepConsts&, cudaStream_t);               \
+                                              const GeneralTopo&, const StepConsts&, cudaStream_t, bool);         \
   template cudaError_t launch_accumulate<T>(int, const void*, const void*, void*, const GeneralTopo&,            \
                                             const StepConsts&, cudaStream_t);                                     \
   template cudaError_t launch_integrate<T>(int, int, float, const void*, const void*, const void*, void*, void*, \

@@ -8,6 +8,7 @@
 // chosen), so the result is bit-identical to the general gather.
 #include <type_traits>
 
+#include "chain_launch.cuh"
 #include "cp_async.cuh"
 #include "face_pair.cuh"
 #include "fastdiv.cuh"
@@ -563,6 +564,10 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
   else
     copy_halo();
 
+  // what was read so far (constants, tables) no step writes
+  chain_wait();
+  chain_next();
+
   // ---- stage the state as pairs: whole rows of EC pairs a round, so a thread
   // keeps its column
   bool slow = false;  // an edge tile with a non-finite state
@@ -869,8 +874,8 @@ int batched_ctas_per_sm_t() {
 
 template <int TH>
 void launch_batched_t(int grid, const ClothDesc* cloths, const int4* work, int parity, const StepConsts& c,
-                      cudaStream_t s, const int* n_work_dev) {
-  k_step_batched<TH><<<grid, Tile<TH>::NT, Tile<TH>::SMEM, s>>>(cloths, work, parity, c, n_work_dev);
+                      cudaStream_t s, const int* n_work_dev, bool chained) {
+  chain_launch(k_step_batched<TH>, grid, Tile<TH>::NT, Tile<TH>::SMEM, s, chained, cloths, work, parity, c, n_work_dev);
 }
 
 }  // namespace
@@ -930,21 +935,21 @@ int batched_ctas_per_sm(int th) {
 }
 
 cudaError_t launch_step_batched(const ClothDesc* cloths, const int4* work, int n_work, int parity,
-                                const StepConsts& c, cudaStream_t s, const int* n_work_dev, int th) {
+                                const StepConsts& c, cudaStream_t s, bool chained, const int* n_work_dev, int th) {
   if (n_work <= 0) return cudaSuccess;
   if (!batch_tile_height_ok(th)) return cudaErrorInvalidValue;
   const cudaError_t ea = prime_step_kernels();
   if (ea != cudaSuccess) return ea;
   switch (th) {
-    case 4: launch_batched_t<4>(n_work, cloths, work, parity, c, s, n_work_dev); break;
-    case 12: launch_batched_t<12>(n_work, cloths, work, parity, c, s, n_work_dev); break;
-    default: launch_batched_t<8>(n_work, cloths, work, parity, c, s, n_work_dev); break;
+    case 4: launch_batched_t<4>(n_work, cloths, work, parity, c, s, n_work_dev, chained); break;
+    case 12: launch_batched_t<12>(n_work, cloths, work, parity, c, s, n_work_dev, chained); break;
+    default: launch_batched_t<8>(n_work, cloths, work, parity, c, s, n_work_dev, chained); break;
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4* vel, const float4* force_in,
-                             float4* pos_out, float4* vel_out, const StepConsts& c, cudaStream_t s) {
+                             float4* pos_out, float4* vel_out, const StepConsts& c, cudaStream_t s, bool chained) {
   const int n = g.rows * g.cols;
   if (n <= 0) return cudaSuccess;
   if (g.variant == 1) {
@@ -963,8 +968,8 @@ cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4*
       const bool has_interior = t.bx1 >= t.bx0 && t.by1 >= t.by0;
       const int n_interior = has_interior ? (t.bx1 - t.bx0 + 1) * (t.by1 - t.by0 + 1) : 0;
       const int n_ring = t.tx * t.ty - n_interior;
-      kernel<<<n_ring + n_interior, threads, smem, s>>>(g.rows, g.cols, t, n_ring, g.params, pos, vel, force_in,
-                                                        pos_out, vel_out, c);
+      chain_launch(kernel, n_ring + n_interior, threads, smem, s, chained, g.rows, g.cols, t, n_ring, g.params, pos, vel,
+                   force_in, pos_out, vel_out, c);
     };
     const long long tiles8 = (long long)((g.cols + kTileW - 1) / kTileW) * ((g.rows + 7) / 8);
     if (tiles8 <= kSms)
