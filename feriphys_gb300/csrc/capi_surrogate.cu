@@ -218,13 +218,13 @@ int ensure_train_scratch(fgb_surrogate* g, int ctas, size_t n_losses) {
 // One Adam step on the rows staged in d_X/d_T.
 int adam_step(fgb_surrogate* g, uint64_t n_rows, float lr, float* d_loss_slot) {
   const int ctas = S::train_ctas(int(n_rows));
-  FGB_CUDA(S::launch_train(g->d_X, g->d_T, int(n_rows), g->d_blob, g->d_partials, ctas, g->d_err, g->stream));
+  FGB_CUDA(S::launch_train(g->d_X, g->d_T, int(n_rows), g->d_blob, g->d_partials, ctas, g->d_err, g->stream, true));
   g->adam_t += 1;
   const double t = double(g->adam_t);
   const float c1 = float(1.0 / (1.0 - std::pow(0.9, t)));
   const float c2 = float(1.0 / (1.0 - std::pow(0.999, t)));
   FGB_CUDA(S::launch_adam(g->d_partials, ctas, g->d_master, g->d_m, g->d_v, lr, 0.9f, 0.999f, 1e-8f, c1, c2,
-                          g->d_blob, d_loss_slot, 1.0f / (3.0f * float(n_rows)), g->stream));
+                          g->d_blob, d_loss_slot, 1.0f / (3.0f * float(n_rows)), g->stream, true));
   g->host_stale = true;
   return FGB_OK;
 }
@@ -807,7 +807,7 @@ int fgb_surrogate_gradients(fgb_surrogate* g, const float* x, const float* t, ui
   const int ctas = S::train_ctas(int(n));
   FGB_CHECK_RC(ensure_train_scratch(g, ctas, 1));
   FGB_CUDA(dgrow(g->d_grad, g->grad_cap, S::kNumParams, sizeof(float)));
-  FGB_CUDA(S::launch_train(g->d_X, g->d_T, int(n), g->d_blob, g->d_partials, ctas, g->d_err, g->stream));
+  FGB_CUDA(S::launch_train(g->d_X, g->d_T, int(n), g->d_blob, g->d_partials, ctas, g->d_err, g->stream, false));
   FGB_CUDA(S::launch_reduce_grad(g->d_partials, ctas, 1.0f / (3.0f * float(n)), g->d_grad, g->d_loss, g->stream));
   std::vector<float> P(S::kNumParams);
   float l = 0.0f;
@@ -938,7 +938,7 @@ int fgb_surrogate_train(fgb_surrogate* g, uint64_t n_steps, uint64_t batch, floa
   for (uint64_t k = 0; k < n_steps; ++k) {
     const uint64_t bseed = seed * 0x2545F4914F6CDD1DULL + k * 0x9E3779B97F4A7C15ULL;
     FGB_CUDA(S::launch_pack_batch(g->d_feat, g->d_tgt, g->count, bseed, int(batch), g->norm, g->d_X, g->d_T,
-                                  g->stream));
+                                  g->stream, k > 0));
     FGB_CHECK_RC(adam_step(g, batch, lr, g->d_loss + k));
   }
   if (losses)

@@ -18,6 +18,7 @@
 //    the CTA and are written out once.
 #include <cuda_bf16.h>
 
+#include "chain_launch.cuh"
 #include "devmath.cuh"
 #include "grid_order.h"
 #include "per_device.h"
@@ -622,6 +623,8 @@ __global__ void __launch_bounds__(kTrThreads, 1)
   }
   __syncthreads();
   tc::fence_after_sync();
+  chain_wait();  // the launches before write the weights and the batch and read the partials
+  chain_next();
   if (lt == 0) {
     tc::mbar_arrive_expect_tx(&bar_w, kBlobBytes);
     tc::bulk_g2s(smem, blob, kBlobBytes, &bar_w);
@@ -823,42 +826,81 @@ __device__ __forceinline__ void blob_store(unsigned char* blob, int p, float w) 
   }
 }
 
-__device__ __forceinline__ float loss_sum(const float* partials, int ctas) {
-  float s = 0.0f;
-  for (int c = 0; c < ctas; ++c) s += partials[size_t(c) * kPartialStride + kNumParams];
-  return s;
-}
+// Sums of 32 columns of the CTAs' partials, each in CTA order.  The block's
+// eight warps fetch the rows w, w + 8, ... into shared memory, all loads of a
+// thread in flight at once (16 MB of partials: one thread per column walking
+// them took 17 us, 9 with the fetch spread out); the first warp then adds.
+// Columns kNumParams and up hold the loss sum.  Returns the thread's column sum
+// (first warp only).
+constexpr int kSumWarps = 8, kSumCols = 32;
+constexpr int kParamBlock = 32 * kSumWarps;
+constexpr int kParamGrid = (kNumParams + 1 + kSumCols - 1) / kSumCols;
+constexpr int kSumMost = 256;  // CTAs whose partials fit (32 KB); launch_train's grid is one per SM
+constexpr int kSumRound = 20;  // loads in flight a thread
 
-// the gradient of parameter p = param_of_partial(q), summed over the CTAs in
-// CTA order (the threads of a block read consecutive partials q)
-__device__ __forceinline__ float grad_sum(const float* partials, int ctas, int q, int p) {
+__device__ __forceinline__ float partial_sums(const float* __restrict__ partials, int ctas,
+                                              float (&buf)[kSumMost][kSumCols]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q = blockIdx.x * kSumCols + lane;
+  const bool ok = q < kPartialStride;
   float g = 0.0f;
-  for (int c = 0; c < ctas; ++c) g += partials[size_t(c) * kPartialStride + q];
-  return param_used(p) ? g : 0.0f;
+  for (int c0 = 0; c0 < ctas; c0 += kSumMost) {
+    const int n = min(ctas - c0, kSumMost);
+    for (int r0 = warp; r0 < n; r0 += kSumWarps * kSumRound) {
+      float x[kSumRound];
+#pragma unroll
+      for (int j = 0; j < kSumRound; ++j) {
+        const int r = r0 + j * kSumWarps;
+        x[j] = ok && r < n ? __ldg(partials + size_t(c0 + r) * kPartialStride + q) : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < kSumRound; ++j) {
+        const int r = r0 + j * kSumWarps;
+        if (r < n) buf[r][lane] = x[j];
+      }
+    }
+    __syncthreads();
+    if (warp == 0)
+#pragma unroll 8
+      for (int r = 0; r < n; ++r) g += buf[r][lane];
+    __syncthreads();
+  }
+  return g;
 }
 
-__global__ void k_reduce_grad(const float* __restrict__ partials, int ctas, float inv_count, float* __restrict__ grad,
-                              float* __restrict__ loss_out) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q == 0 && loss_out) loss_out[0] = loss_sum(partials, ctas) * inv_count;
+__global__ void __launch_bounds__(kParamBlock)
+    k_reduce_grad(const float* __restrict__ partials, int ctas, float inv_count, float* __restrict__ grad,
+                  float* __restrict__ loss_out) {
+  __shared__ float buf[kSumMost][kSumCols];
+  const float g = partial_sums(partials, ctas, buf);
+  const int q = blockIdx.x * kSumCols + threadIdx.x;
+  if (threadIdx.x >= 32) return;
+  if (q == kNumParams && loss_out) loss_out[0] = g * inv_count;
   if (q >= kNumParams) return;
   const int p = param_of_partial(q);
-  grad[p] = grad_sum(partials, ctas, q, p);
+  grad[p] = param_used(p) ? g : 0.0f;
 }
 
-__global__ void k_adam(const float* __restrict__ partials, int ctas, float* __restrict__ master, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float beta1, float beta2, float eps, float c1, float c2,
-                       unsigned char* __restrict__ blob, float* __restrict__ loss_out, float inv_count) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q == 0 && loss_out) loss_out[0] = loss_sum(partials, ctas) * inv_count;
-  if (q >= kNumParams) return;
-  const int p = param_of_partial(q);
-  const float g = grad_sum(partials, ctas, q, p);
-  const float mm = beta1 * m[p] + (1.0f - beta1) * g;
-  const float vv = beta2 * v[p] + (1.0f - beta2) * (g * g);
+__global__ void __launch_bounds__(kParamBlock)
+    k_adam(const float* __restrict__ partials, int ctas, float* __restrict__ master, float* __restrict__ m,
+           float* __restrict__ v, float lr, float beta1, float beta2, float eps, float c1, float c2,
+           unsigned char* __restrict__ blob, float* __restrict__ loss_out, float inv_count) {
+  __shared__ float buf[kSumMost][kSumCols];
+  chain_wait();
+  chain_next();
+  const int q = blockIdx.x * kSumCols + threadIdx.x;
+  const bool mine = threadIdx.x < 32 && q < kNumParams;
+  const int p = mine ? param_of_partial(q) : 0;
+  const float m0 = m[p], v0 = v[p], w0 = master[p];
+  const float sum = partial_sums(partials, ctas, buf);
+  if (threadIdx.x < 32 && q == kNumParams && loss_out) loss_out[0] = sum * inv_count;
+  if (!mine) return;
+  const float g = param_used(p) ? sum : 0.0f;
+  const float mm = beta1 * m0 + (1.0f - beta1) * g;
+  const float vv = beta2 * v0 + (1.0f - beta2) * (g * g);
   m[p] = mm;
   v[p] = vv;
-  float w = master[p] - lr * (mm * c1) / (sqrtf(vv * c2) + eps);
+  float w = w0 - lr * (mm * c1) / (sqrtf(vv * c2) + eps);
   if (!param_used(p)) w = 0.0f;
   master[p] = w;
   blob_store(blob, p, w);
@@ -927,21 +969,54 @@ __global__ void k_features(const SurCloth* __restrict__ cloth, const Tile* __res
   for (int k = 0; k < kFeat; ++k) out[size_t(v) * kFeat + k] = f[k];
 }
 
-__global__ void k_pack_batch(const float* __restrict__ feat, const float* __restrict__ tgt, long long count,
-                             uint64_t seed, int n_rows, const Norm nm, unsigned char* __restrict__ X,
-                             float* __restrict__ T) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_rows) return;
-  const long long row = (long long)(mix64(seed ^ (uint64_t(b) * 0x9E3779B97F4A7C15ULL)) % uint64_t(count));
-  const float* f = feat + row * kRawStride;
-  float x[kFeat];
+// A warp takes 32 rows of the batch: each lane draws one of them, then half a
+// warp at a time reads a row (16 float4, whole lines) and writes it
+// standardised as bf16.  (A thread per row reading its 54 floats one by one
+// took 18.3 us for 65,536 rows, 8.8 like this.)  The batch buffers are free when
+// it starts (chain_launch.cuh: the launch before it has waited for the training
+// that read them), so it waits only before it ends: the training after it
+// needs the optimizer step before it.
+__global__ void __launch_bounds__(128)
+    k_pack_batch(const float* __restrict__ feat, const float* __restrict__ tgt, long long count, uint64_t seed,
+                 int n_rows, const __grid_constant__ Norm nm, unsigned char* __restrict__ X, float* __restrict__ T) {
+  static_assert(kRawStride == 64 && kIn == 64, "a row is 16 float4");
+  chain_next();
+  const int lane = threadIdx.x & 31, base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
+  const int b = base + lane;  // n_rows is a multiple of 128
+  if (base < n_rows) {
+    const long long row = (long long)(mix64(seed ^ (uint64_t(b) * 0x9E3779B97F4A7C15ULL)) % uint64_t(count));
+    const float4 t = __ldg(reinterpret_cast<const float4*>(tgt) + row);
+    const int k = 4 * (lane & 15);
+    float mean[4], inv[4];
 #pragma unroll
-  for (int k = 0; k < kFeat; ++k) x[k] = f[k];
-  store_input_row(X + size_t(b >> 7) * 16384, b & 127, x, true, nm);
-  const float4 t = reinterpret_cast<const float4*>(tgt)[row];
-  reinterpret_cast<float4*>(T)[b] = make_float4((t.x - nm.out_mean[0]) / nm.out_std[0],
-                                                (t.y - nm.out_mean[1]) / nm.out_std[1],
-                                                (t.z - nm.out_mean[2]) / nm.out_std[2], 0.0f);
+    for (int e = 0; e < 4; ++e) {
+      mean[e] = k + e < kFeat ? nm.in_mean[k + e] : 0.0f;
+      inv[e] = k + e < kFeat ? nm.in_inv_std[k + e] : 0.0f;
+    }
+#pragma unroll 1
+    for (int i0 = 0; i0 < 16; i0 += 8) {
+      float4 f[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const long long r = __shfl_sync(0xffffffffu, row, 2 * (i0 + i) + (lane >> 4));
+        f[i] = __ldg(reinterpret_cast<const float4*>(feat + r * kRawStride + k));
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int o = base + 2 * (i0 + i) + (lane >> 4);
+        const float x[4] = {f[i].x, f[i].y, f[i].z, f[i].w};
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = k + e < kFeat ? (x[e] - mean[e]) * inv[e] : 0.0f;
+        *reinterpret_cast<uint2*>(X + size_t(o >> 7) * 16384 + tc::blk_off(kIn, o & 127, k)) =
+            make_uint2(pack_bf2(y[0], y[1]), pack_bf2(y[2], y[3]));
+      }
+    }
+    reinterpret_cast<float4*>(T)[b] = make_float4((t.x - nm.out_mean[0]) / nm.out_std[0],
+                                                  (t.y - nm.out_mean[1]) / nm.out_std[1],
+                                                  (t.z - nm.out_mean[2]) / nm.out_std[2], 0.0f);
+  }
+  chain_wait();
 }
 
 __global__ void k_pack_rows(const float* __restrict__ x, const float* __restrict__ t, int n, int n_pad,
@@ -1284,29 +1359,27 @@ int train_ctas(int n_rows) {
 }
 
 cudaError_t launch_train(const void* X, const float* T, int n_rows, const void* blob, float* partials, int ctas,
-                         int* err, cudaStream_t s) {
+                         int* err, cudaStream_t s, bool chained) {
   const int n_tiles = n_rows / kTile;
   if (n_tiles <= 0 || ctas <= 0) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem);
   if (e != cudaSuccess) return e;
   const float dscale = 2.0f / (3.0f * float(n_rows));
-  k_train<<<ctas, kTrThreads, kTrSmem, s>>>(static_cast<const unsigned char*>(X), T, n_tiles,
-                                     static_cast<const unsigned char*>(blob), partials, dscale, err);
-  return cudaGetLastError();
+  return chain_launch(k_train, ctas, kTrThreads, kTrSmem, s, chained, static_cast<const unsigned char*>(X), T, n_tiles,
+                      static_cast<const unsigned char*>(blob), partials, dscale, err);
 }
 
 cudaError_t launch_reduce_grad(const float* partials, int ctas, float inv_count, float* grad, float* loss_out,
                                cudaStream_t s) {
-  k_reduce_grad<<<(kNumParams + 255) / 256, 256, 0, s>>>(partials, ctas, inv_count, grad, loss_out);
+  k_reduce_grad<<<kParamGrid, kParamBlock, 0, s>>>(partials, ctas, inv_count, grad, loss_out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_adam(const float* partials, int ctas, float* master, float* m, float* v, float lr, float beta1,
                         float beta2, float eps, float c1, float c2, void* blob, float* loss_out, float inv_count,
-                        cudaStream_t s) {
-  k_adam<<<(kNumParams + 255) / 256, 256, 0, s>>>(partials, ctas, master, m, v, lr, beta1, beta2, eps, c1, c2,
-                                                  static_cast<unsigned char*>(blob), loss_out, inv_count);
-  return cudaGetLastError();
+                        cudaStream_t s, bool chained) {
+  return chain_launch(k_adam, kParamGrid, kParamBlock, 0, s, chained, partials, ctas, master, m, v, lr, beta1, beta2, eps,
+                      c1, c2, static_cast<unsigned char*>(blob), loss_out, inv_count);
 }
 
 cudaError_t launch_pack_blob(const float* master, void* blob, cudaStream_t s) {
@@ -1336,11 +1409,10 @@ cudaError_t launch_features(const SurCloth* cloth, const Tile* tiles, int n_tile
 }
 
 cudaError_t launch_pack_batch(const float* feat, const float* tgt, long long count, uint64_t seed, int n_rows,
-                              const Norm& norm, void* X, float* T, cudaStream_t s) {
+                              const Norm& norm, void* X, float* T, cudaStream_t s, bool chained) {
   if (n_rows <= 0 || count <= 0) return cudaErrorInvalidValue;
-  k_pack_batch<<<(n_rows + 127) / 128, 128, 0, s>>>(feat, tgt, count, seed, n_rows, norm,
-                                                    static_cast<unsigned char*>(X), T);
-  return cudaGetLastError();
+  return chain_launch(k_pack_batch, (n_rows + 127) / 128, 128, 0, s, chained, feat, tgt, count, seed, n_rows, norm,
+                      static_cast<unsigned char*>(X), T);
 }
 
 cudaError_t launch_pack_rows(const float* x, const float* t, int n, int n_pad, void* X, float* T, cudaStream_t s) {

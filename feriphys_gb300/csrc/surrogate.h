@@ -104,8 +104,9 @@ cudaError_t launch_forward(const void* X, int n_rows, const void* blob, float* Y
 // Fused forward + backward of the mean squared error over n_rows rows (a
 // multiple of 128): per-CTA gradient partials [ctas][kPartialStride] (the
 // loss sum at kNumParams).  ctas <= min(#SMs, n_rows / 128).
+// chained (here and below): chain_launch.cuh.
 cudaError_t launch_train(const void* X, const float* T, int n_rows, const void* blob, float* partials, int ctas,
-                         int* err, cudaStream_t s);
+                         int* err, cudaStream_t s, bool chained);
 int train_ctas(int n_rows);
 
 // Sum of the partials in CTA order; then either only the gradient (grad !=
@@ -116,7 +117,7 @@ cudaError_t launch_reduce_grad(const float* partials, int ctas, float inv_count,
                                cudaStream_t s);
 cudaError_t launch_adam(const float* partials, int ctas, float* master, float* m, float* v, float lr, float beta1,
                         float beta2, float eps, float c1, float c2, void* blob, float* loss_out, float inv_count,
-                        cudaStream_t s);
+                        cudaStream_t s, bool chained);
 // master (padded f32) -> blob.
 cudaError_t launch_pack_blob(const float* master, void* blob, cudaStream_t s);
 
@@ -134,7 +135,7 @@ cudaError_t launch_features(const SurCloth* cloth, const Tile* tiles, int n_tile
 // Training batch: n_rows rows drawn from the first `count` ring rows (seeded
 // hash), standardised, X as bf16 blocked, T[n][4] f32.
 cudaError_t launch_pack_batch(const float* feat, const float* tgt, long long count, uint64_t seed, int n_rows,
-                              const Norm& norm, void* X, float* T, cudaStream_t s);
+                              const Norm& norm, void* X, float* T, cudaStream_t s, bool chained);
 // Standardised host rows (x[n][54], t[n][3] or null) -> X blocked, T[n][4];
 // rows n..n_pad-1 are zero.
 cudaError_t launch_pack_rows(const float* x, const float* t, int n, int n_pad, void* X, float* T, cudaStream_t s);
