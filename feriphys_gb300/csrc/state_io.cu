@@ -73,25 +73,38 @@ __global__ void k_set_pins(int n, const uint8_t* __restrict__ pinned, Vec4<T>* _
 
 inline int nb(int n) { return (n + 255) / 256; }
 
-// The same conversions for f32 state with the Stateful rows moved as
-// coalesced 16-byte chunks through shared memory (256 points = 10 KB per
-// block); the rows may sit in device memory or, mapped, in pinned host memory,
-// which the kernel then reads or writes across the host link directly.  The
-// row pointer must be 16-byte aligned.
+// The same conversions for f32 state with the Stateful rows moved in coalesced
+// chunks through shared memory (256 points = 10 KB per block); the rows may
+// sit in device memory or, mapped, in pinned host memory, which the kernel
+// then reads or writes across the host link directly.  Chunk: what the row
+// pointer is aligned to, float4, float2 (rows from an odd point on) or float.
+// (A thread per row took 31 us to write 13,500 points from an odd point on
+// across the link, 6 in chunks.)
 constexpr int kIoBlock = 256;
 
+template <class Chunk>
 __global__ void __launch_bounds__(kIoBlock) k_unpack_staged(int n, const float* __restrict__ pts,
                                                             const uint8_t* __restrict__ pinned,
                                                             float4* __restrict__ pos, float4* __restrict__ vel,
                                                             float4* __restrict__ force) {
+  constexpr int W = sizeof(Chunk) / 4, EACH = 10 / W + (10 % W != 0);
   __shared__ __align__(16) float buf[10 * kIoBlock];
   const int first = blockIdx.x * kIoBlock;
   const int cnt = min(kIoBlock, n - first);
   const int nf = 10 * cnt;
   const float* src = pts + 10 * size_t(first);
-  for (int k = threadIdx.x; k < nf / 4; k += kIoBlock)
-    reinterpret_cast<float4*>(buf)[k] = reinterpret_cast<const float4*>(src)[k];
-  for (int k = (nf / 4) * 4 + threadIdx.x; k < nf; k += kIoBlock) buf[k] = src[k];
+  Chunk x[EACH];
+#pragma unroll
+  for (int j = 0; j < EACH; ++j) {
+    const int k = threadIdx.x + j * kIoBlock;
+    if (k < nf / W) x[j] = reinterpret_cast<const Chunk*>(src)[k];
+  }
+#pragma unroll
+  for (int j = 0; j < EACH; ++j) {
+    const int k = threadIdx.x + j * kIoBlock;
+    if (k < nf / W) reinterpret_cast<Chunk*>(buf)[k] = x[j];
+  }
+  for (int k = (nf / W) * W + threadIdx.x; k < nf; k += kIoBlock) buf[k] = src[k];
   __syncthreads();
   const int t = threadIdx.x;
   if (t >= cnt) return;
@@ -102,9 +115,11 @@ __global__ void __launch_bounds__(kIoBlock) k_unpack_staged(int n, const float* 
   if (force) force[i] = make_float4(p[7], p[8], p[9], 0.0f);
 }
 
+template <class Chunk>
 __global__ void __launch_bounds__(kIoBlock) k_pack_staged(int n, const float4* __restrict__ pos,
                                                           const float4* __restrict__ vel,
                                                           const float4* __restrict__ force, float* __restrict__ pts) {
+  constexpr int W = sizeof(Chunk) / 4;
   __shared__ __align__(16) float buf[10 * kIoBlock];
   const int first = blockIdx.x * kIoBlock;
   const int cnt = min(kIoBlock, n - first);
@@ -122,9 +137,8 @@ __global__ void __launch_bounds__(kIoBlock) k_pack_staged(int n, const float4* _
   __syncthreads();
   const int nf = 10 * cnt;
   float* dst = pts + 10 * size_t(first);
-  for (int k = t; k < nf / 4; k += kIoBlock)
-    reinterpret_cast<float4*>(dst)[k] = reinterpret_cast<const float4*>(buf)[k];
-  for (int k = (nf / 4) * 4 + t; k < nf; k += kIoBlock) dst[k] = buf[k];
+  for (int k = t; k < nf / W; k += kIoBlock) reinterpret_cast<Chunk*>(dst)[k] = reinterpret_cast<const Chunk*>(buf)[k];
+  for (int k = (nf / W) * W + t; k < nf; k += kIoBlock) dst[k] = buf[k];
 }
 
 template <class T>
@@ -162,9 +176,11 @@ template <class T>
 cudaError_t launch_unpack(int n, const float* pts, const uint8_t* pinned, void* pos, void* vel, void* force,
                           cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(pts) & 15) == 0) {
-    k_unpack_staged<<<(n + kIoBlock - 1) / kIoBlock, kIoBlock, 0, s>>>(
-        n, pts, pinned, static_cast<float4*>(pos), static_cast<float4*>(vel), static_cast<float4*>(force));
+  if (sizeof(T) == 4) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(pts);
+    auto k = (a & 15) == 0 ? k_unpack_staged<float4> : ((a & 7) == 0 ? k_unpack_staged<float2> : k_unpack_staged<float>);
+    k<<<(n + kIoBlock - 1) / kIoBlock, kIoBlock, 0, s>>>(n, pts, pinned, static_cast<float4*>(pos),
+                                                         static_cast<float4*>(vel), static_cast<float4*>(force));
     return cudaGetLastError();
   }
   k_unpack<T><<<nb(n), 256, 0, s>>>(n, pts, pinned, static_cast<Vec4<T>*>(pos), static_cast<Vec4<T>*>(vel),
@@ -175,9 +191,12 @@ cudaError_t launch_unpack(int n, const float* pts, const uint8_t* pinned, void* 
 template <class T>
 cudaError_t launch_pack_f32(int n, const void* pos, const void* vel, const void* force, float* pts, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(pts) & 15) == 0) {
-    k_pack_staged<<<(n + kIoBlock - 1) / kIoBlock, kIoBlock, 0, s>>>(
-        n, static_cast<const float4*>(pos), static_cast<const float4*>(vel), static_cast<const float4*>(force), pts);
+  if (sizeof(T) == 4) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(pts);
+    auto k = (a & 15) == 0 ? k_pack_staged<float4> : ((a & 7) == 0 ? k_pack_staged<float2> : k_pack_staged<float>);
+    k<<<(n + kIoBlock - 1) / kIoBlock, kIoBlock, 0, s>>>(n, static_cast<const float4*>(pos),
+                                                         static_cast<const float4*>(vel),
+                                                         static_cast<const float4*>(force), pts);
     return cudaGetLastError();
   }
   k_pack<T, float><<<nb(n), 256, 0, s>>>(n, static_cast<const Vec4<T>*>(pos), static_cast<const Vec4<T>*>(vel),

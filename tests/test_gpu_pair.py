@@ -187,3 +187,23 @@ def test_split_step_any_valence(fgb, orc, bits, valence):
         osim.step(1)
     g, o = m.get_points()[:, 1:7].astype(np.float64), om.get_points()[:, 1:7].astype(np.float64)
     assert np.abs(g - o).max() / np.abs(o).max() <= 1e-6  # five steps of f32 rounding; the terms are O(1) of the state
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 1000])
+def test_exchange_at_any_offset(fgb, n, offset, pinned):
+    """Stateful rows from and to a buffer at every alignment a float array can
+    have, at the edges of the conversion's 256-point blocks, unchanged."""
+    import torch
+
+    rng = np.random.default_rng(n + offset)
+    m = fgb.SpringyMesh.new(rng.normal(0, 1, (n, 3)).astype(np.float32), [], 0.01 * n, 1.0, 1.0)
+    sim = fgb.Simulation.new([m], [])
+    sim.step(0)
+    flat = lambda: torch.zeros(10 * n + offset, pin_memory=pinned).numpy()[offset:].reshape(n, 10)  # noqa: E731
+    src, dst = flat(), flat()
+    src[:] = rng.normal(0, 1, (n, 10)).astype(np.float32)
+    m.set_points(src)
+    got = m.get_points(dst)
+    assert got.tobytes() == src.tobytes()
