@@ -3,6 +3,7 @@
 // coarse rollout with the energy/strain checks and the fine-step fallback.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -81,7 +82,8 @@ struct fgb_surrogate {
   size_t grad_cap = 0;
   double* d_stats = nullptr;
   size_t stats_cap = 0;
-  int* d_err = nullptr;
+  S::RolloutCtl* d_ctl = nullptr;
+  int* d_err = nullptr;  // &d_ctl->err
   // coarse-step tables
   S::SurCloth* d_cloths = nullptr;
   size_t cloths_cap = 0;
@@ -100,7 +102,7 @@ struct fgb_surrogate {
   int groups = 4;
   // checked rollout decided on the device (per cloth: accepted energy, margin
   // scale, verdict; per batch cloth: work-list range, mesh index, compacted
-  // position; counters: this step's failures, fallback items, running total)
+  // position; the stop word and counters)
   float* d_e_old = nullptr;
   size_t e_old_cap = 0;
   double* d_e_ref = nullptr;
@@ -109,9 +111,6 @@ struct fgb_surrogate {
   size_t fail_cap = 0;
   int* d_bidx = nullptr;  // 4 x n_batch: off, cnt, mesh, dst
   size_t bidx_cap = 0;
-  int* d_counts = nullptr;  // [0] failures this step, [1] fallback items
-  unsigned long long* d_total = nullptr;
-  cudaStream_t side = nullptr;  // captures the fallback body
 };
 
 namespace {
@@ -182,15 +181,16 @@ int sync_host_master(fgb_surrogate* g) {
   return FGB_OK;
 }
 
+int tensor_core_error(fgb_surrogate* g, cudaStream_t st) {
+  FGB_CUDA(cudaMemsetAsync(g->d_err, 0, sizeof(int), st));
+  return fail(FGB_ECHECK, "a tensor-core kernel gave up waiting for its copies or MMAs");
+}
+
 int check_err(fgb_surrogate* g, cudaStream_t st) {
   int e = 0;
   FGB_CUDA(cudaMemcpyAsync(&e, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   FGB_CUDA(cudaStreamSynchronize(st));
-  if (e) {
-    FGB_CUDA(cudaMemsetAsync(g->d_err, 0, sizeof(int), st));
-    return fail(FGB_ECHECK, "a tensor-core kernel gave up waiting for its copies or MMAs");
-  }
-  return FGB_OK;
+  return e ? tensor_core_error(g, st) : FGB_OK;
 }
 
 // Standardised host rows -> packed bf16 tiles (and targets) on the device.
@@ -292,13 +292,21 @@ void add_tiles(int cloth, S::SurCloth& c, std::vector<S::Tile>& tiles) {
   for (int k = 0; k < c.ntiles; ++k) tiles.push_back(make_int2(cloth, k * S::kTile));
 }
 
+// Waits for a stream's work at the end of a scope: declared after the host
+// tables that the work may still be reading.
+struct Drain {
+  cudaStream_t st;
+  ~Drain() { cudaStreamSynchronize(st); }
+};
+
+// wait = false: the caller keeps the tables until the stream is done with them.
 int upload_tables(fgb_surrogate* g, const std::vector<S::SurCloth>& cl, const std::vector<S::Tile>& tiles,
-                  cudaStream_t st) {
+                  cudaStream_t st, bool wait) {
   FGB_CUDA(dgrow(g->d_cloths, g->cloths_cap, cl.size(), sizeof(S::SurCloth)));
   FGB_CUDA(dgrow(g->d_tiles, g->tiles_cap, tiles.size(), sizeof(S::Tile)));
   FGB_CUDA(cudaMemcpyAsync(g->d_cloths, cl.data(), cl.size() * sizeof(S::SurCloth), cudaMemcpyHostToDevice, st));
   FGB_CUDA(cudaMemcpyAsync(g->d_tiles, tiles.data(), tiles.size() * sizeof(S::Tile), cudaMemcpyHostToDevice, st));
-  FGB_CUDA(cudaStreamSynchronize(st));
+  if (wait) FGB_CUDA(cudaStreamSynchronize(st));
   return FGB_OK;
 }
 
@@ -329,7 +337,7 @@ void mesh_wind(const fgb_sim* s, const fgb_mesh* m, float w[3]) {
 }
 
 int build_sim_tables(fgb_surrogate* g, fgb_sim* s, float T, long long vbase0, std::vector<S::SurCloth>& cl,
-                     std::vector<S::Tile>& tiles, cudaStream_t st) {
+                     std::vector<S::Tile>& tiles, cudaStream_t st, bool wait = true) {
   cl.clear();
   tiles.clear();
   long long vb = vbase0;
@@ -341,7 +349,7 @@ int build_sim_tables(fgb_surrogate* g, fgb_sim* s, float T, long long vbase0, st
     add_tiles(int(i), cl.back(), tiles);
     vb += (long long)s->meshes[i]->topo.n;
   }
-  return upload_tables(g, cl, tiles, st);
+  return upload_tables(g, cl, tiles, st, wait);
 }
 
 int run_check(fgb_surrogate* g, fgb_sim* s, int n_tiles, int parity, std::vector<float2>& out, cudaStream_t st) {
@@ -416,7 +424,13 @@ int fine_fallback(fgb_surrogate* g, fgb_sim* s, const std::vector<int>& failing,
 
 constexpr int kHostDecides = 1;  // not an error: run the host-decided loop instead
 
-// Inputs of the graph-built rollout that stay fixed for one call.
+// Steps launched ahead of their verdicts: so many at first, twice as many
+// after each run without a failure up to the most, and one after a failure.
+// A run ends with a host wait (about 12 us); a launch that a failure before it
+// has stopped costs about 6 us a step.
+constexpr uint64_t kAheadFirst = 8, kAheadMost = 32;
+
+// Inputs of a checked rollout that stay fixed for one call.
 struct Rollout {
   uint32_t ratio = 1;
   int n_tiles = 0, n_cloths = 0, n_batch = 0;
@@ -425,11 +439,11 @@ struct Rollout {
   float growth = 0.0f, abs_margin = 0.0f, max_strain = 0.0f;
 };
 
-// The fallback of the cloths that failed this step (the body of the graph's
-// conditional): the same fine steps as fine_fallback, with the failing set
-// and the compacted work list made on the device, then a re-check whose
-// energies the failing cloths accept.  Launched on `bs` while it captures.
-int capture_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, cudaStream_t bs) {
+// The fallback of the cloths that failed a step from buffers [par]: the same
+// fine steps as fine_fallback, with the failing set and the compacted work
+// list made on the device, then a re-check whose energies the failing cloths
+// accept.
+int device_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, cudaStream_t st) {
   if (s->batch.empty()) {
     fgb_mesh* m = s->meshes[0];
     const fgb::GridTopo gt{int(m->topo.rows), int(m->topo.cols), m->d_grid, 0};
@@ -439,11 +453,11 @@ int capture_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, c
     for (uint32_t j = 0; j < ro.ratio; ++j, a ^= 1)
       FGB_CUDA(fgb::launch_step_grid(gt, static_cast<const float4*>(m->pos[a]), static_cast<const float4*>(m->vel[a]),
                                      nullptr, static_cast<float4*>(m->pos[a ^ 1]), static_cast<float4*>(m->vel[a ^ 1]),
-                                     mc, bs, false));
+                                     mc, st, j > 0));
     if (a != (par ^ 1)) {
       const size_t bytes = size_t(m->topo.n) * sizeof(float4);
-      FGB_CUDA(cudaMemcpyAsync(m->pos[par ^ 1], m->pos[a], bytes, cudaMemcpyDeviceToDevice, bs));
-      FGB_CUDA(cudaMemcpyAsync(m->vel[par ^ 1], m->vel[a], bytes, cudaMemcpyDeviceToDevice, bs));
+      FGB_CUDA(cudaMemcpyAsync(m->pos[par ^ 1], m->pos[a], bytes, cudaMemcpyDeviceToDevice, st));
+      FGB_CUDA(cudaMemcpyAsync(m->vel[par ^ 1], m->vel[a], bytes, cudaMemcpyDeviceToDevice, st));
     }
   } else {
     const int nb = ro.n_batch;
@@ -452,91 +466,33 @@ int capture_fallback(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, c
     int* mesh = cnt + nb;
     int* dst = mesh + nb;
     FGB_CUDA(S::launch_fallback_tables(s->d_desc, mesh, nb, g->d_fail, off, cnt, s->d_work, g->d_fdesc, dst,
-                                       g->d_fwork, g->d_counts + 1, bs));
+                                       g->d_fwork, &g->d_ctl->items, st));
     int from = par;
     if ((ro.ratio & 1u) == 0) {
-      FGB_CUDA(S::launch_copy_unskipped(g->d_fdesc, nb, par, bs));
+      FGB_CUDA(S::launch_copy_unskipped(g->d_fdesc, nb, par, st));
       from = par ^ 1;
     }
     for (uint32_t j = 0; j < ro.ratio; ++j)
-      FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, s->n_work, from ^ int(j & 1u), ro.fine, bs,
-                                        false, g->d_counts + 1, s->tile_h));
+      FGB_CUDA(fgb::launch_step_batched(g->d_fdesc, g->d_fwork, s->n_work, from ^ int(j & 1u), ro.fine, st,
+                                        j > 0, &g->d_ctl->items, s->tile_h));
   }
   FGB_CUDA(S::launch_check(g->d_cloths, g->d_tiles, ro.n_tiles, ro.n_cloths, par ^ 1, ro.gforce, g->d_tile_chk,
-                           g->d_cloth_chk, bs));
-  FGB_CUDA(S::launch_accept(g->d_cloth_chk, ro.n_cloths, g->d_fail, g->d_e_old, bs));
+                           g->d_cloth_chk, st));
+  FGB_CUDA(S::launch_accept(g->d_cloth_chk, ro.n_cloths, g->d_fail, g->d_e_old, st));
   return FGB_OK;
 }
 
-// One coarse step from buffers [par] as a graph: surrogate step, check,
-// verdicts, and the fallback body under an IF conditional the verdict
-// kernel sets.
-int capture_checked_step(fgb_surrogate* g, fgb_sim* s, const Rollout& ro, int par, cudaStream_t st,
-                         cudaGraphExec_t* out) {
-  FGB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  int rc = FGB_OK;
-  cudaError_t e = cudaSuccess;
-  do {
-    if ((e = cudaMemsetAsync(g->d_counts, 0, sizeof(int), st)) != cudaSuccess) break;
-    if ((e = S::launch_sur_step(g->d_cloths, g->d_tiles, ro.n_tiles, par, g->d_blob, g->norm, ro.coarse, g->groups, 0,
-                                g->d_err, st)) != cudaSuccess)
-      break;
-    if ((e = S::launch_check(g->d_cloths, g->d_tiles, ro.n_tiles, ro.n_cloths, par ^ 1, ro.gforce, g->d_tile_chk,
-                             g->d_cloth_chk, st)) != cudaSuccess)
-      break;
-    if ((e = S::launch_decide(g->d_cloth_chk, ro.n_cloths, g->d_e_old, g->d_e_ref, ro.growth, ro.abs_margin,
-                              ro.max_strain, g->d_fail, g->d_counts, st)) != cudaSuccess)
-      break;
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    if ((e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, nullptr, nullptr, nullptr)) != cudaSuccess) break;
-    cudaGraphConditionalHandle h;
-    if ((e = cudaGraphConditionalHandleCreate(&h, cg, 0, cudaGraphCondAssignDefault)) != cudaSuccess) break;
-    if ((e = S::launch_set_fallback(h, g->d_counts, g->d_total, st)) != cudaSuccess) break;
-    if ((e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, nullptr, &nd)) != cudaSuccess) break;
-    cudaGraphNodeParams cp{};  // every member zero
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cn;
-    if ((e = cudaGraphAddNode(&cn, cg, deps, nullptr, nd, &cp)) != cudaSuccess) break;
-    if ((e = cudaStreamUpdateCaptureDependencies(st, &cn, nullptr, 1, cudaStreamSetCaptureDependencies)) !=
-        cudaSuccess)
-      break;
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    if ((e = cudaStreamBeginCaptureToGraph(g->side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-        cudaSuccess)
-      break;
-    rc = capture_fallback(g, s, ro, par, g->side);
-    cudaGraph_t body_out = nullptr;
-    const cudaError_t eb = cudaStreamEndCapture(g->side, &body_out);
-    if (rc == FGB_OK && eb != cudaSuccess) e = eb;
-  } while (false);
-  cudaGraph_t graph = nullptr;
-  const cudaError_t ee = cudaStreamEndCapture(st, &graph);
-  if (rc == FGB_OK && e == cudaSuccess) e = ee;
-  if (rc != FGB_OK || e != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    cudaGetLastError();
-    return rc != FGB_OK ? rc : fail(FGB_ECUDA, cudaGetErrorString(e));
-  }
-  e = cudaGraphInstantiate(out, graph, 0);
-  cudaGraphDestroy(graph);
-  FGB_CUDA(e);
-  return FGB_OK;
-}
-
-// The checked rollout with every decision on the device: one graph launch
-// per coarse step and one host wait at the end.  Decisions, fallbacks and
-// states equal the host-decided loop's (the same kernels; the verdict is the
-// same double-precision test).  Returns kHostDecides before touching the
-// state when the graph cannot be built (the caller then decides on the host).
+// The checked rollout with every decision on the device: steps, checks and
+// verdicts are launched some steps ahead, the first failing verdict turns
+// what was launched after it into launches that do nothing, and the host, at
+// the end of the run, adds that step's fallback and goes on after it.
+// Decisions, fallbacks and states equal the host-decided loop's (the same
+// kernels; the verdict is the same double-precision test).  Returns
+// kHostDecides before touching the state for a batch whose work list is not
+// one contiguous range a cloth.
 int rollout_on_device(fgb_surrogate* g, fgb_sim* s, uint32_t ratio, uint64_t n_coarse,
                       const fgb_surrogate_check* chk, int n_tiles, const fgb::StepConsts& cst,
-                      const std::vector<float2>& e_old, const std::vector<double>& e_ref, cudaStream_t st,
+                      const std::vector<double>& e_ref, cudaStream_t st,
                       uint64_t* n_fallbacks) {
   Rollout ro;
   ro.ratio = ratio;
@@ -580,49 +536,49 @@ int rollout_on_device(fgb_surrogate* g, fgb_sim* s, uint32_t ratio, uint64_t n_c
   FGB_CUDA(dgrow(g->d_e_old, g->e_old_cap, size_t(nc), sizeof(float)));
   FGB_CUDA(dgrow(g->d_e_ref, g->e_ref_cap, size_t(nc), sizeof(double)));
   FGB_CUDA(dgrow(g->d_fail, g->fail_cap, size_t(nc), sizeof(int)));
-  if (!g->d_counts) FGB_CUDA(cudaMalloc(&g->d_counts, 2 * sizeof(int)));
-  if (!g->d_total) FGB_CUDA(cudaMalloc(&g->d_total, sizeof(unsigned long long)));
-  if (!g->side) FGB_CUDA(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
-  std::vector<float> e0(nc);
-  for (int c = 0; c < nc; ++c) e0[c] = e_old[c].x;
-  FGB_CUDA(cudaMemcpyAsync(g->d_e_old, e0.data(), nc * sizeof(float), cudaMemcpyHostToDevice, st));
+  FGB_CUDA(dgrow(g->d_tile_chk, g->tile_chk_cap, size_t(n_tiles), sizeof(float2)));
+  FGB_CUDA(dgrow(g->d_cloth_chk, g->cloth_chk_cap, size_t(nc), sizeof(float2)));
+  const Drain drain{st};  // the tables' uploads
   FGB_CUDA(cudaMemcpyAsync(g->d_e_ref, e_ref.data(), nc * sizeof(double), cudaMemcpyHostToDevice, st));
   if (nb > 0)
     FGB_CUDA(cudaMemcpyAsync(g->d_bidx, bidx.data(), bidx.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-  FGB_CUDA(cudaMemsetAsync(g->d_total, 0, sizeof(unsigned long long), st));
-  FGB_CUDA(cudaStreamSynchronize(st));  // the host tables must outlive their upload
-  FGB_CUDA(S::prime_sur_step(g->groups));
-  FGB_CUDA(fgb::prime_step_kernels());
+  FGB_CUDA(cudaMemsetAsync(g->d_ctl, 0, offsetof(S::RolloutCtl, err), st));
+  // the state the call starts from: accepted as it is
+  FGB_CUDA(S::launch_tile_check(g->d_cloths, g->d_tiles, n_tiles, s->parity, ro.gforce, g->d_tile_chk, nullptr, st));
+  FGB_CUDA(S::launch_verdict(g->d_cloths, g->d_tile_chk, nc, g->d_e_old, g->d_e_ref, ro.growth, ro.abs_margin,
+                             ro.max_strain, g->d_fail, g->d_ctl, 0, st));
 
-  cudaGraphExec_t exec[2] = {nullptr, nullptr};
-  const int p0 = s->parity;
-  int rc = capture_checked_step(g, s, ro, p0, st, &exec[p0]);
-  if (rc == FGB_OK && n_coarse > 1) rc = capture_checked_step(g, s, ro, p0 ^ 1, st, &exec[p0 ^ 1]);
-  if (rc != FGB_OK) {
-    for (cudaGraphExec_t x : exec)
-      if (x) cudaGraphExecDestroy(x);
-    cudaGetLastError();
-    return kHostDecides;
-  }
-  cudaError_t e = cudaSuccess;
-  for (uint64_t k = 0; k < n_coarse && e == cudaSuccess; ++k) {
-    e = cudaGraphLaunch(exec[s->parity], st);
-    if (e != cudaSuccess) break;
-    s->parity ^= 1;
-    for (fgb_mesh* m : s->meshes) {
-      m->cur = s->parity;
-      m->has_force = false;
-      m->staged = false;
+  S::RolloutCtl ctl{};
+  uint64_t ahead = kAheadFirst;
+  for (uint64_t k = 0; k < n_coarse;) {
+    const int m = int(std::min<uint64_t>(ahead, n_coarse - k));
+    int par = s->parity;
+    for (int j = 0; j < m; ++j, par ^= 1) {
+      FGB_CUDA(S::launch_sur_step(g->d_cloths, g->d_tiles, ro.n_tiles, par, g->d_blob, g->norm, ro.coarse, g->groups, 0,
+                                  g->d_err, st, j > 0, &g->d_ctl->stop));
+      FGB_CUDA(S::launch_tile_check(g->d_cloths, g->d_tiles, ro.n_tiles, par ^ 1, ro.gforce, g->d_tile_chk,
+                                    &g->d_ctl->stop, st));
+      FGB_CUDA(S::launch_verdict(g->d_cloths, g->d_tile_chk, ro.n_cloths, g->d_e_old, g->d_e_ref, ro.growth,
+                                 ro.abs_margin, ro.max_strain, g->d_fail, g->d_ctl, j + 1, st));
+    }
+    FGB_CUDA(cudaMemcpyAsync(&ctl, g->d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st));
+    FGB_CUDA(cudaStreamSynchronize(st));
+    const int done = ctl.stop > 0 ? ctl.stop : m;
+    if (ctl.stop > 0) {
+      FGB_CUDA(cudaMemsetAsync(&g->d_ctl->stop, 0, sizeof(int), st));
+      FGB_CHECK_RC(device_fallback(g, s, ro, s->parity ^ ((done - 1) & 1), st));
+    }
+    ahead = ctl.stop > 0 ? 1 : std::min(2 * ahead, kAheadMost);
+    k += uint64_t(done);
+    s->parity ^= done & 1;
+    for (fgb_mesh* mesh : s->meshes) {
+      mesh->cur = s->parity;
+      mesh->has_force = false;
+      mesh->staged = false;
     }
   }
-  unsigned long long total = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&total, g->d_total, sizeof(total), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  for (cudaGraphExec_t x : exec)
-    if (x) cudaGraphExecDestroy(x);
-  FGB_CUDA(e);
-  if (n_fallbacks) *n_fallbacks = total;
-  return FGB_OK;
+  if (n_fallbacks) *n_fallbacks = ctl.total;
+  return ctl.err ? tensor_core_error(g, st) : FGB_OK;
 }
 
 }  // namespace
@@ -644,11 +600,14 @@ int fgb_surrogate_new(uint64_t seed, fgb_surrogate** out) {
         cudaMalloc(&g->d_master, S::kNumParams * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&g->d_m, S::kNumParams * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&g->d_v, S::kNumParams * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&g->d_blob, S::kBlobBytes) != cudaSuccess || cudaMalloc(&g->d_err, sizeof(int)) != cudaSuccess ||
-        cudaMemset(g->d_err, 0, sizeof(int)) != cudaSuccess || cudaMemset(g->d_blob, 0, S::kBlobBytes) != cudaSuccess) {
+        cudaMalloc(&g->d_blob, S::kBlobBytes) != cudaSuccess ||
+        cudaMalloc(&g->d_ctl, sizeof(S::RolloutCtl)) != cudaSuccess ||
+        cudaMemset(g->d_ctl, 0, sizeof(S::RolloutCtl)) != cudaSuccess ||
+        cudaMemset(g->d_blob, 0, S::kBlobBytes) != cudaSuccess) {
       rc = fail(FGB_ECUDA, "device allocation failed");
       break;
     }
+    g->d_err = &g->d_ctl->err;
     std::vector<float> flat(kFlat, 0.0f);
     Rng r{seed};
     float* q = flat.data();
@@ -696,7 +655,6 @@ int fgb_surrogate_destroy(fgb_surrogate* g) {
   dfree(g->d_loss);
   dfree(g->d_grad);
   dfree(g->d_stats);
-  dfree(g->d_err);
   dfree(g->d_cloths);
   dfree(g->d_tiles);
   dfree(g->d_tile_chk);
@@ -708,9 +666,7 @@ int fgb_surrogate_destroy(fgb_surrogate* g) {
   dfree(g->d_e_ref);
   dfree(g->d_fail);
   dfree(g->d_bidx);
-  dfree(g->d_counts);
-  dfree(g->d_total);
-  if (g->side) cudaStreamDestroy(g->side);
+  dfree(g->d_ctl);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
   return FGB_OK;
@@ -776,7 +732,7 @@ int fgb_surrogate_features(fgb_surrogate* g, fgb_mesh* m, float coarse_dt, const
   std::vector<S::SurCloth> cl{make_cloth(m, coarse_dt, w, 0)};
   std::vector<S::Tile> tiles;
   add_tiles(0, cl[0], tiles);
-  FGB_CHECK_RC(upload_tables(g, cl, tiles, m->stream));
+  FGB_CHECK_RC(upload_tables(g, cl, tiles, m->stream, true));
   const size_t n = m->topo.n;
   FGB_CUDA(dgrow(g->d_out, g->out_cap, n * S::kFeat, sizeof(float)));
   FGB_CUDA(S::launch_features(g->d_cloths, g->d_tiles, int(tiles.size()), m->cur, g->d_out, m->stream));
@@ -961,7 +917,8 @@ int fgb_sim_step_surrogate(fgb_sim* s, fgb_surrogate* g, uint32_t ratio, uint64_
   align_parity(s);
   std::vector<S::SurCloth> cl;
   std::vector<S::Tile> tiles;
-  FGB_CHECK_RC(build_sim_tables(g, s, T, 0, cl, tiles, st));
+  const Drain drain{st};
+  FGB_CHECK_RC(build_sim_tables(g, s, T, 0, cl, tiles, st, false));
   const int n_tiles = int(tiles.size());
   fgb_config cc = s->cfg;
   cc.dt = T;
@@ -976,22 +933,23 @@ int fgb_sim_step_surrogate(fgb_sim* s, fgb_surrogate* g, uint32_t ratio, uint64_
     for (size_t c = 0; c < s->meshes.size(); ++c)
       e_ref[c] = double(s->meshes[c]->topo.n) * gmag * double(mesh_spacing(s->meshes[c]));
   }
+  // the margin's scale (with the first energy added) is fixed for the whole
+  // call, so the allowed growth is linear in the number of coarse steps, never
+  // compounding
+  if (checks && s->graphs) {
+    const int rd = rollout_on_device(g, s, ratio, n_coarse, chk, n_tiles, cst, e_ref, st, n_fallbacks);
+    if (rd != kHostDecides) return rd;
+  }
   if (checks) {
     FGB_CHECK_RC(run_check(g, s, n_tiles, s->parity, e_old, st));
-    // the margin's scale is fixed for the whole call, so the allowed growth is
-    // linear in the number of coarse steps, never compounding
     for (size_t c = 0; c < s->meshes.size(); ++c) e_ref[c] += std::fabs(double(e_old[c].x));
-  }
-  if (checks && s->graphs) {
-    const int rd = rollout_on_device(g, s, ratio, n_coarse, chk, n_tiles, cst, e_old, e_ref, st, n_fallbacks);
-    if (rd != kHostDecides) return rd == FGB_OK ? check_err(g, st) : rd;
   }
   uint64_t fallbacks = 0;
   std::vector<int> failing;
   for (uint64_t k = 0; k < n_coarse; ++k) {
     const int par = s->parity;
     FGB_CUDA(S::launch_sur_step(g->d_cloths, g->d_tiles, n_tiles, par, g->d_blob, g->norm, cst, g->groups, 0,
-                                g->d_err, st));
+                                g->d_err, st, !checks && k > 0));
     if (checks) {
       FGB_CHECK_RC(run_check(g, s, n_tiles, par ^ 1, e_new, st));
       failing.clear();

@@ -18,7 +18,7 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // kernel<<<blocks, threads, smem, s>>>(args...), chained to the launch before
-// it when `chained`.  Not for the body of a conditional graph node.
+// it when `chained`.
 template <class... P, class... A>
 cudaError_t chain_launch(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t s, bool chained,
                          A... args) {

@@ -54,7 +54,8 @@ template <class T>
 cudaError_t launch_zero4(int n, void* a, cudaStream_t s);
 
 // chained: the launch may overlap the end of the one before it in the stream
-// (chain_launch.cuh); false in the body of a conditional graph node.
+// (chain_launch.cuh); false where that one writes what a step reads besides
+// the state (cloth tables, work items).
 cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4* vel, const float4* force_in,
                              float4* pos_out, float4* vel_out, const StepConsts& c, cudaStream_t s, bool chained);
 

@@ -416,13 +416,19 @@ __device__ __forceinline__ bool mlp_tile(unsigned char* act, const unsigned char
 
 // ---- inference: the coarse step --------------------------------------------
 
+// A checked rollout launches some steps ahead of their verdicts; the first
+// that fails sets *stop, and what was launched after it then does nothing.
+__device__ __forceinline__ bool stopped(const int* stop) {
+  return stop && *static_cast<const volatile int*>(stop) != 0;
+}
+
 // G groups of 128 * H threads; a group takes one 128-vertex tile at a time,
 // H threads per vertex row (H = 2: each computes half of the row's features
 // and half of its hidden columns, so twice the warps hide the latencies).
 template <int G, int H>
 __global__ void __launch_bounds__(128 * G * H, 1)
     k_sur_step(const SurCloth* __restrict__ cloths, const Tile* __restrict__ tiles, int n_tiles, int parity,
-               const unsigned char* __restrict__ blob, const Norm norm, const StepConsts cst, int* err) {
+               const unsigned char* __restrict__ blob, const Norm norm, const StepConsts cst, int* err, const int* stop) {
   static_assert(H == 1 || H == 2, "one or two threads per row");
   constexpr int NT = 128 * H;
   constexpr uint32_t kCols = G == 1 ? 128 : (G == 2 ? 256 : 512);  // a power of two >= 128 G
@@ -450,6 +456,12 @@ __global__ void __launch_bounds__(128 * G * H, 1)
     tc::bulk_g2s(smem, blob, kBlobBytes, &bar_w);
   }
   bool ok = __syncthreads_and(tc::mbar_wait(&bar_w, 0)) != 0;
+  // the step before: from here on its states may be read and its inputs
+  // overwritten (262,144 vertices, unchecked: 56.1 us a step unchained, 52.9
+  // with the tables' and the weights' loads before this wait; 4,096: 18.6, 14.9)
+  chain_wait();
+  chain_next();
+  if (stopped(stop)) n_tiles = 0;
   const uint32_t tmem = tslot + uint32_t(g * 128);
   const uint32_t lane_off = uint32_t((row >> 5) * 32) << 16;
   unsigned char* act = smem + kBlobSmem + g * 32768;
@@ -1079,27 +1091,42 @@ __global__ void k_stats(const float* __restrict__ feat, const float* __restrict_
 
 // ---- checks ----------------------------------------------------------------
 
+// A vertex's share of its cloth's energy and its own struts' largest strain,
+// summed per tile.  One load deep and then bound by latency, so the constants
+// (which no step writes) are read before the wait for the step checked.
 __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ cloths, const Tile* __restrict__ tiles,
-                                               int n_tiles, int parity, float3 gf, float2* __restrict__ tile_out) {
+                                               int parity, float3 gf, float2* __restrict__ tile_out, const int* stop) {
   __shared__ float2 red[4];
   const int t = blockIdx.x;
-  if (t >= n_tiles) return;
   const Tile w = tiles[t];
   const SurCloth& c = cloths[w.x];
   const int R = c.rows, C = c.cols, n = R * C;
   const int v = w.y + threadIdx.x;
+  const int r = v / C, col = v % C;
   const float4* __restrict__ P = c.pos[parity];
   const float4* __restrict__ Vl = c.vel[parity];
-  float E = 0.0f, S = 0.0f;
-  if (v < n) {
-    const int r = v / C, col = v % C;
-    const float4 p = P[v], vel = Vl[v];
+  float k[5], L[5];
+  bool has[5];
+  {
     const float* __restrict__ prm = c.params + grid::param_rec(r, col, C);
     const int pc = col % 16, lane = (col / 16) % 2;
+#pragma unroll
+    for (int kind = 0; kind < 5; ++kind) {
+      has[kind] = v < n && grid::owned_exists(kind, r, col, R, C);
+      k[kind] = has[kind] ? prm[64 * kind + 4 * pc + lane] : 0.0f;
+      L[kind] = has[kind] ? prm[320 + 32 * kind + 2 * pc + lane] : 1.0f;
+    }
+  }
+  chain_wait();
+  chain_next();
+  if (stopped(stop)) return;
+  float E = 0.0f, S = 0.0f;
+  if (v < n) {
+    const float4 p = P[v], vel = Vl[v];
     E = 0.5f * p.w * ((vel.x * vel.x + vel.y * vel.y) + vel.z * vel.z) - ((gf.x * p.x + gf.y * p.y) + gf.z * p.z);
 #pragma unroll
     for (int kind = 0; kind < 5; ++kind) {
-      if (!grid::owned_exists(kind, r, col, R, C)) continue;
+      if (!has[kind]) continue;
       int a = v, b;
       switch (kind) {
         case grid::KH: b = v + 1; break;
@@ -1111,11 +1138,9 @@ __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ clot
       const float4 pa = a == v ? p : P[a], pb = P[b];
       const float dx = pb.x - pa.x, dy = pb.y - pa.y, dz = pb.z - pa.z;
       const float d = sqrtf((dx * dx + dy * dy) + dz * dz);
-      const float k = prm[64 * kind + 4 * pc + lane];
-      const float L = prm[320 + 32 * kind + 2 * pc + lane];
-      const float e = d - L;
-      E += 0.5f * k * (e * e);
-      S = fmaxf(S, fabsf(e / L));
+      const float e = d - L[kind];
+      E += 0.5f * k[kind] * (e * e);
+      S = fmaxf(S, fabsf(e / L[kind]));
     }
     if (!isfinite(E)) E = __int_as_float(0x7f800000);
     if (!(S == S)) S = __int_as_float(0x7f800000);
@@ -1136,12 +1161,8 @@ __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ clot
 // run, whatever the number of tiles).
 constexpr int kReduceBlock = 256;
 
-__global__ void __launch_bounds__(kReduceBlock) k_check_reduce(const SurCloth* __restrict__ cloths,
-                                                               const float2* __restrict__ tile_out,
-                                                               float2* __restrict__ cloth_out) {
-  __shared__ float2 sh[kReduceBlock];
-  const int c = blockIdx.x;
-  const SurCloth& cl = cloths[c];
+__device__ __forceinline__ float2 cloth_sum(const SurCloth& cl, const float2* __restrict__ tile_out,
+                                            float2 (&sh)[kReduceBlock]) {
   float E = 0.0f, S = 0.0f;
   for (int k = threadIdx.x; k < cl.ntiles; k += kReduceBlock) {
     const float2 e = tile_out[cl.tile0 + k];
@@ -1158,7 +1179,15 @@ __global__ void __launch_bounds__(kReduceBlock) k_check_reduce(const SurCloth* _
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) cloth_out[c] = sh[0];
+  return sh[0];
+}
+
+__global__ void __launch_bounds__(kReduceBlock) k_check_reduce(const SurCloth* __restrict__ cloths,
+                                                               const float2* __restrict__ tile_out,
+                                                               float2* __restrict__ cloth_out) {
+  __shared__ float2 sh[kReduceBlock];
+  const float2 e = cloth_sum(cloths[blockIdx.x], tile_out, sh);
+  if (threadIdx.x == 0) cloth_out[blockIdx.x] = e;
 }
 
 __global__ void k_copy_unskipped(const ClothDesc* __restrict__ cloths, int from) {
@@ -1173,17 +1202,37 @@ __global__ void k_copy_unskipped(const ClothDesc* __restrict__ cloths, int from)
 
 // ---- device-side decisions of a checked rollout ------------------------------
 
-// Per cloth: the rollout's energy/strain test of the state a coarse step
-// produced (cloth_out) against the last accepted energy e_old and the margin
-// growth * e_ref + abs, evaluated in double exactly as the host form does.
-// Passing cloths accept their new energy; fail[c] is the verdict; n_fail
-// counts this step's failures.
-__global__ void k_decide(const float2* __restrict__ cloth_out, int n_cloths, float* __restrict__ e_old,
-                         const double* __restrict__ e_ref, float growth, float abs_margin, float max_strain,
-                         int* __restrict__ fail, int* __restrict__ n_fail) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_cloths) return;
-  const float2 o = cloth_out[c];
+// One block per cloth: its check's sums (as k_check_reduce), then the rollout's
+// energy/strain test of the state a coarse step produced against the last
+// accepted energy e_old and the margin growth * e_ref + abs, evaluated in
+// double exactly as the host form does.  Passing cloths accept their new
+// energy; fail[c] is the verdict.  The last block to finish stops the steps
+// launched after this one if any cloth failed (ctl->stop = step), and adds the
+// failures to the call's total.
+//
+// 262,144 vertices, microseconds a checked coarse step (without the check 53):
+// 83 as a graph of step, check, reduction, decision, and a conditional node
+// with the fallback; 76 with one verdict kernel and chained launches in it;
+// 63 launched ahead without a graph (the conditional node alone is 11; the
+// two graphs' capture and instantiation, per call, took 190 more).  4,096
+// vertices: 43 and 22 (unchecked 19 and 15).
+__global__ void __launch_bounds__(kReduceBlock)
+    k_verdict(const SurCloth* __restrict__ cloths, const float2* __restrict__ tile_out, float* __restrict__ e_old,
+              double* __restrict__ e_ref, float growth, float abs_margin, float max_strain,
+              int* __restrict__ fail, RolloutCtl* ctl, int step) {
+  __shared__ float2 sh[kReduceBlock];
+  const int c = blockIdx.x;
+  chain_wait();
+  chain_next();
+  // (this launch's own stop is set after every block has counted itself below)
+  if (stopped(&ctl->stop)) return;
+  const float2 o = cloth_sum(cloths[c], tile_out, sh);
+  if (threadIdx.x != 0) return;
+  if (step == 0) {  // the state the call starts from
+    e_old[c] = o.x;
+    e_ref[c] += fabs(double(o.x));
+    return;
+  }
   const double E0 = e_old[c], E1 = o.x, S1 = o.y;
   const double margin = double(growth) * e_ref[c] + double(abs_margin);
   const bool ok = isfinite(E1) && isfinite(S1) && (E1 <= E0 + margin) && (S1 <= double(max_strain));
@@ -1191,16 +1240,15 @@ __global__ void k_decide(const float2* __restrict__ cloth_out, int n_cloths, flo
   if (ok)
     e_old[c] = o.x;
   else
-    atomicAdd(n_fail, 1);
-}
-
-// One thread: the graph's fallback conditional from this step's failure
-// count, which is also added to the call's running total.
-__global__ void k_set_fallback(cudaGraphConditionalHandle h, const int* __restrict__ n_fail,
-                               unsigned long long* __restrict__ total) {
-  const int v = *n_fail;
-  cudaGraphSetConditional(h, v > 0 ? 1u : 0u);
-  *total += (unsigned long long)v;
+    atomicAdd(&ctl->failing, 1);
+  __threadfence();
+  if (atomicAdd(&ctl->judged, 1) != int(gridDim.x) - 1) return;
+  const int v = atomicExch(&ctl->failing, 0);
+  ctl->judged = 0;
+  if (v > 0) {
+    ctl->total += (unsigned long long)v;
+    ctl->stop = step;
+  }
 }
 
 // The batched fallback's cloth table (the batch's, with skip = !fail and no
@@ -1298,7 +1346,7 @@ cudaError_t sur_step_attr() {
 
 template <int G, int H>
 cudaError_t sur_step_g(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, const void* blob,
-                       const Norm& norm, const StepConsts& consts, int ctas, int* err, cudaStream_t s) {
+                       const Norm& norm, const StepConsts& consts, int ctas, int* err, cudaStream_t s, bool chained, const int* stop) {
   const int smem = kBlobSmem + G * 32768;
   const cudaError_t e = sur_step_attr<G, H>();
   if (e != cudaSuccess) return e;
@@ -1306,9 +1354,8 @@ cudaError_t sur_step_g(const SurCloth* cloths, const Tile* tiles, int n_tiles, i
   const int cap = ctas > 0 ? ctas : sm_count();
   if (grid > cap) grid = cap;
   if (grid < 1) return cudaSuccess;
-  k_sur_step<G, H><<<grid, 128 * G * H, smem, s>>>(cloths, tiles, n_tiles, parity,
-                                                   static_cast<const unsigned char*>(blob), norm, consts, err);
-  return cudaGetLastError();
+  return chain_launch(k_sur_step<G, H>, grid, 128 * G * H, smem, s, chained, cloths, tiles, n_tiles, parity,
+                      static_cast<const unsigned char*>(blob), norm, consts, err, stop);
 }
 
 }  // namespace
@@ -1318,26 +1365,15 @@ constexpr int kRowThreads = 2;
 
 int sur_step_max_ctas(int) { return sm_count(); }
 
-cudaError_t prime_sur_step(int groups) {
-  switch (groups) {
-    case 1: return sur_step_attr<1, kRowThreads>();
-    case 2: return sur_step_attr<2, kRowThreads>();
-    case 3: return sur_step_attr<3, kRowThreads>();
-    default: return sur_step_attr<4, kRowThreads>();
-  }
-}
-
-
-
 cudaError_t launch_sur_step(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, const void* blob,
                             const Norm& norm, const StepConsts& consts, int groups, int ctas, int* err,
-                            cudaStream_t s) {
+                            cudaStream_t s, bool chained, const int* stop) {
   if (n_tiles <= 0) return cudaSuccess;
   switch (groups) {
-    case 1: return sur_step_g<1, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s);
-    case 2: return sur_step_g<2, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s);
-    case 3: return sur_step_g<3, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s);
-    default: return sur_step_g<4, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s);
+    case 1: return sur_step_g<1, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s, chained, stop);
+    case 2: return sur_step_g<2, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s, chained, stop);
+    case 3: return sur_step_g<3, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s, chained, stop);
+    default: return sur_step_g<4, kRowThreads>(cloths, tiles, n_tiles, parity, blob, norm, consts, ctas, err, s, chained, stop);
   }
 }
 
@@ -1430,23 +1466,23 @@ cudaError_t launch_stats(const float* feat, const float* tgt, long long count, d
 cudaError_t launch_check(const SurCloth* cloths, const Tile* tiles, int n_tiles, int n_cloths, int parity,
                          float3 gforce, float2* tile_out, float2* cloth_out, cudaStream_t s) {
   if (n_tiles <= 0) return cudaSuccess;
-  k_check<<<n_tiles, kTile, 0, s>>>(cloths, tiles, n_tiles, parity, gforce, tile_out);
+  k_check<<<n_tiles, kTile, 0, s>>>(cloths, tiles, parity, gforce, tile_out, nullptr);
   if (n_cloths > 0) k_check_reduce<<<n_cloths, kReduceBlock, 0, s>>>(cloths, tile_out, cloth_out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_decide(const float2* cloth_out, int n_cloths, float* e_old, const double* e_ref, float growth,
-                          float abs_margin, float max_strain, int* fail, int* n_fail, cudaStream_t s) {
-  if (n_cloths <= 0) return cudaSuccess;
-  k_decide<<<(n_cloths + 255) / 256, 256, 0, s>>>(cloth_out, n_cloths, e_old, e_ref, growth, abs_margin, max_strain,
-                                                  fail, n_fail);
-  return cudaGetLastError();
+cudaError_t launch_tile_check(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, float3 gforce,
+                              float2* tile_out, const int* stop, cudaStream_t s) {
+  if (n_tiles <= 0) return cudaSuccess;
+  return chain_launch(k_check, n_tiles, kTile, 0, s, true, cloths, tiles, parity, gforce, tile_out, stop);
 }
 
-cudaError_t launch_set_fallback(cudaGraphConditionalHandle h, const int* n_fail, unsigned long long* total,
-                                cudaStream_t s) {
-  k_set_fallback<<<1, 1, 0, s>>>(h, n_fail, total);
-  return cudaGetLastError();
+cudaError_t launch_verdict(const SurCloth* cloths, const float2* tile_out, int n_cloths, float* e_old,
+                           double* e_ref, float growth, float abs_margin, float max_strain, int* fail,
+                           RolloutCtl* ctl, int step, cudaStream_t s) {
+  if (n_cloths <= 0) return cudaErrorInvalidValue;
+  return chain_launch(k_verdict, n_cloths, kReduceBlock, 0, s, true, cloths, tile_out, e_old, e_ref, growth, abs_margin,
+                      max_strain, fail, ctl, step);
 }
 
 cudaError_t launch_fallback_tables(const ClothDesc* desc, const int* bmesh, int n_batch, const int* fail,

@@ -91,10 +91,11 @@ using Tile = int2;
 // Coarse step of every listed tile: features, MLP on the tensor cores,
 // v' = v + dv, p' = p + (v + v') T / 2 (the mean velocity over the step), collision response against the obstacles
 // (consts: dt = T), pinned vertices unchanged.  groups = 128-thread groups per
-// CTA (2 or 4), ctas = persistent CTAs (0: one per tile group).
+// CTA (2 or 4), ctas = persistent CTAs (0: one per tile group).  stop: a word that
+// turns the launch into one that does nothing when it is not 0 (RolloutCtl), or null.
 cudaError_t launch_sur_step(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, const void* blob,
                             const Norm& norm, const StepConsts& consts, int groups, int ctas, int* err,
-                            cudaStream_t s);
+                            cudaStream_t s, bool chained, const int* stop = nullptr);
 int sur_step_max_ctas(int groups);
 
 // Network outputs (standardised units, bias included) for standardised
@@ -159,29 +160,36 @@ cudaError_t launch_check(const SurCloth* cloths, const Tile* tiles, int n_tiles,
 // the pre-step state before stepping from it).
 cudaError_t launch_copy_unskipped(const ClothDesc* cloths, int n_cloths, int from, cudaStream_t s);
 
-// Device-side decisions of a checked rollout (no host round trip per coarse
-// step).  launch_decide: per cloth, the energy/strain test of cloth_out
-// against e_old and the margin growth * e_ref + abs (in double, as the host
-// form), fail[c] = verdict, e_old[c] = E for passing cloths, n_fail += the
-// failures.  launch_set_fallback: one thread sets the graph conditional h to
-// (*n_fail > 0) and adds *n_fail to *total.  launch_fallback_tables: the
-// batched fallback's cloth table (skip = !fail[bmesh[b]], no forces) and the
-// failing cloths' work items (cloth b owns items [off[b], off[b] + cnt[b])
-// of `work`) compacted in list order into fwork, their count in *n_out
-// (dst: n_batch ints of scratch).  launch_accept: e_old[c] = cloth_out[c].x
-// for every failing cloth.
-cudaError_t launch_decide(const float2* cloth_out, int n_cloths, float* e_old, const double* e_ref, float growth,
-                          float abs_margin, float max_strain, int* fail, int* n_fail, cudaStream_t s);
-cudaError_t launch_set_fallback(cudaGraphConditionalHandle h, const int* n_fail, unsigned long long* total,
-                                cudaStream_t s);
+// A checked rollout's steps are launched ahead of their verdicts.  In device
+// memory, zero at the start of a call up to `err`:
+struct RolloutCtl {
+  int stop;                  // 0, or the `step` of the first verdict that failed: later launches do nothing
+  int failing, judged;       // the running verdict's counters, 0 between verdicts
+  int items;                 // work items of the fallback
+  unsigned long long total;  // cloths that failed so far in the call
+  int err;                   // (not cleared) a tensor-core kernel gave up waiting
+};
+
+// launch_tile_check: the check's sums of every tile (launch_check without the
+// reduction).  launch_verdict: per cloth, the tiles' sum and the energy/strain
+// test against e_old and the margin growth * e_ref + abs (in double, as the
+// host form), fail[c] = verdict, e_old[c] = E for passing cloths; ctl as above
+// (step > 0).  step 0 accepts the state a call starts from: e_old[c] = E,
+// e_ref[c] += |E|.  Both chained to the launch before them.
+// launch_fallback_tables: the batched fallback's cloth table (skip =
+// !fail[bmesh[b]], no forces) and the failing cloths' work items (cloth b owns
+// items [off[b], off[b] + cnt[b]) of `work`) compacted in list order into
+// fwork, their count in *n_out (dst: n_batch ints of scratch).  launch_accept:
+// e_old[c] = cloth_out[c].x for every failing cloth.
+cudaError_t launch_tile_check(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, float3 gforce,
+                              float2* tile_out, const int* stop, cudaStream_t s);
+cudaError_t launch_verdict(const SurCloth* cloths, const float2* tile_out, int n_cloths, float* e_old,
+                           double* e_ref, float growth, float abs_margin, float max_strain, int* fail,
+                           RolloutCtl* ctl, int step, cudaStream_t s);
 cudaError_t launch_fallback_tables(const ClothDesc* desc, const int* bmesh, int n_batch, const int* fail,
                                    const int* off, const int* cnt, const int4* work, ClothDesc* fdesc, int* dst,
                                    int4* fwork, int* n_out, cudaStream_t s);
 cudaError_t launch_accept(const float2* cloth_out, int n_cloths, const int* fail, float* e_old, cudaStream_t s);
-
-// Sets the launch attributes of the coarse-step kernels (call before a
-// stream capture that launches them).
-cudaError_t prime_sur_step(int groups);
 
 }  // namespace sur
 }  // namespace fgb

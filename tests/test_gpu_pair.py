@@ -207,3 +207,29 @@ def test_exchange_at_any_offset(fgb, n, offset, pinned):
     m.set_points(src)
     got = m.get_points(dst)
     assert got.tobytes() == src.tobytes()
+
+
+@pytest.mark.parametrize("steps", [1, 8, 9, 25, 70])
+def test_checked_steps_launched_ahead(fgb, steps):
+    """The checked rollout launches runs of 8, 16, 32 coarse steps ahead of
+    their verdicts, and single ones after a failure: whether no step fails,
+    some do (at the ends of runs and inside them) or all do, the counts and
+    the states are those of the loop that waits for each verdict."""
+    from feriphys_gb300 import workloads as W
+
+    batch = W.c2(n_cloths=3, lo=6, hi=40, seed=2, dt=1.0 / 6000.0)
+    sur = fgb.Surrogate.new(21)
+    chk = fgb.SurrogateCheck.make(energy_growth=1e-3, energy_abs=1e-7, max_strain=0.5)
+    counts = []
+    for scale in (1e-4, *np.geomspace(1e-2, 1e-1, 7), 100.0):
+        sur.set_normalization(np.zeros(54), np.ones(54), np.zeros(3), np.full(3, scale))
+        got = []
+        for ahead in (True, False):
+            sim, meshes, _ = W.build_batch(batch, fgb)
+            sim.set_graphs(ahead)
+            got.append((sim.step_surrogate(sur, 3, steps, chk), [m.get_points() for m in meshes]))
+        assert got[0][0] == got[1][0], scale
+        for a, b in zip(got[0][1], got[1][1]):
+            assert np.array_equal(a, b), scale
+        counts.append(got[0][0])
+    assert len(set(counts)) > 1, counts
