@@ -4,6 +4,11 @@
 // are visible.  chain_next, after the wait, lets the step after this one be
 // placed in turn (after the wait, so that at most one step is ahead).
 //
+// What the launch before writes is read by ordinary loads (its pointers are
+// not __restrict__, no __ldg): the read-only path is for data that stays as it
+// is from a launch's first block to its last, and the first blocks may be
+// there before the last write.
+//
 // What it saves is the gap between dependent launches, most of a small step:
 // 32 x 32 cloth 6.2 -> 4.1 us a step, 157 x 211 6.2 -> 4.5, 500 x 500 16.4 ->
 // 13.6, 1024 x 1024 51.3 -> 47.5, 24 cloths of 16..48 vertices a side (in a

@@ -57,8 +57,8 @@ __device__ __forceinline__ void add_strut(V3<T>& F, V3<T> P, V3<T> V, V3<T> Po, 
   }
 }
 template <class T>
-__device__ __forceinline__ V3<T> face_term(int i0, int i1, int i2, int corner, const Vec4<T>* __restrict__ pos,
-                                           const Vec4<T>* __restrict__ vel, V3<T> wind, const StepConsts& c) {
+__device__ __forceinline__ V3<T> face_term(int i0, int i1, int i2, int corner, const Vec4<T>* pos,
+                                           const Vec4<T>* vel, V3<T> wind, const StepConsts& c) {
   const V3<T> x0 = xyz<T>(pos[i0]), x1 = xyz<T>(pos[i1]), x2 = xyz<T>(pos[i2]);
   const V3<T> v0 = xyz<T>(vel[i0]), v1 = xyz<T>(vel[i1]), v2 = xyz<T>(vel[i2]);
   const V3<T> total = face_total_force<T>(x0, x1, x2, v0, v1, v2, wind, T(c.neg_drag), T(c.neg_lift));
@@ -84,8 +84,8 @@ __device__ __forceinline__ void strut_word(const GeneralTopo& t, int e, int& off
 
 // Strut terms of vertex v added to F in strut order.
 template <class T, int FORM>
-__device__ __forceinline__ V3<T> gather_struts(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* __restrict__ pos,
-                                               const Vec4<T>* __restrict__ vel, const GeneralTopo& t) {
+__device__ __forceinline__ V3<T> gather_struts(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* pos,
+                                               const Vec4<T>* vel, const GeneralTopo& t) {
   const int s_beg = t.strut_off[v], s_end = t.strut_off[v + 1];
   if constexpr (FORM != 0) {
     int own = t.own_off[v];  // owner position of v's next role-0 strut
@@ -109,8 +109,8 @@ __device__ __forceinline__ V3<T> gather_struts(int v, V3<T> P, V3<T> V, V3<T> F,
 
 // The share of v in its face incidence e (s_beg: v's first strut incidence).
 template <class T, int FORM>
-__device__ __forceinline__ V3<T> face_share(int v, int e, int s_beg, const Vec4<T>* __restrict__ pos,
-                                            const Vec4<T>* __restrict__ vel, const GeneralTopo& t, V3<T> wind,
+__device__ __forceinline__ V3<T> face_share(int v, int e, int s_beg, const Vec4<T>* pos,
+                                            const Vec4<T>* vel, const GeneralTopo& t, V3<T> wind,
                                             const StepConsts& c) {
   if constexpr (FORM != 0) {
     const uint32_t h = __ldg(t.face_word + e);
@@ -129,8 +129,8 @@ __device__ __forceinline__ V3<T> face_share(int v, int e, int s_beg, const Vec4<
 }
 
 template <class T, int FORM>
-__device__ __forceinline__ V3<T> gather_forces(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* __restrict__ pos,
-                                               const Vec4<T>* __restrict__ vel, const GeneralTopo& t,
+__device__ __forceinline__ V3<T> gather_forces(int v, V3<T> P, V3<T> V, V3<T> F, const Vec4<T>* pos,
+                                               const Vec4<T>* vel, const GeneralTopo& t,
                                                const StepConsts& c) {
   const V3<T> wind{T(c.wind[0]), T(c.wind[1]), T(c.wind[2])};
   F = gather_struts<T, FORM>(v, P, V, F, pos, vel, t);
@@ -153,7 +153,7 @@ __device__ __forceinline__ void flag_nonfinite(bool bad, unsigned* flags) {
 template <class T> constexpr int kStepBlock = sizeof(T) == 4 ? 256 : 32;
 template <class T, int FORM>
 __global__ void __launch_bounds__(kStepBlock<T>, sizeof(T) == 4 ? 4 : 1)
-    k_step_general(int n, const Vec4<T>* __restrict__ pos, const Vec4<T>* __restrict__ vel,
+    k_step_general(int n, const Vec4<T>* pos, const Vec4<T>* vel,
                    const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
                    GeneralTopo t, StepConsts c) {
   chain_wait();
@@ -197,7 +197,7 @@ template <> struct SplitShape<double> { static constexpr int NF = 6, PER = 1; };
 
 template <class T, int FORM>
 __global__ void __launch_bounds__(32 * (SplitShape<T>::NF + 1))
-    k_step_split(int n, const Vec4<T>* __restrict__ pos, const Vec4<T>* __restrict__ vel,
+    k_step_split(int n, const Vec4<T>* pos, const Vec4<T>* vel,
                  const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
                  GeneralTopo t, StepConsts c) {
   constexpr int NF = SplitShape<T>::NF, PER = SplitShape<T>::PER, SLOTS = NF * PER;

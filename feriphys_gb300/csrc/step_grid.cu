@@ -496,7 +496,7 @@ __host__ __device__ __forceinline__ bool grid_tile(const TileSplit& t, int n_rin
 // One tile of one cloth; edge: some neighbour of a tile vertex may not exist.
 template <int TH>
 __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int C, const float* __restrict__ params,
-                                          const float4* __restrict__ pos, const float4* __restrict__ vel,
+                                          const float4* pos, const float4* vel,
                                           const float4* __restrict__ force_in, float4* __restrict__ pos_out,
                                           float4* __restrict__ vel_out, const StepConsts& c, V3<float> wind,
                                           unsigned* flags) {
@@ -589,8 +589,8 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
           P[k][l] = outside_pos(row, sc + l * kPairW);
           V[k][l] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           if (ok) {
-            P[k][l] = __ldg(src_p + (k * RPR * C + l * kPairW));
-            V[k][l] = __ldg(src_v + (k * RPR * C + l * kPairW));
+            P[k][l] = src_p[k * RPR * C + l * kPairW];
+            V[k][l] = src_v[k * RPR * C + l * kPairW];
           }
           slow |= !(finite3(xyz<float>(P[k][l])) && finite3(xyz<float>(V[k][l])));
         }
@@ -601,8 +601,8 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
         if (sr < RPR && sr + k * RPR < T::EH)
 #pragma unroll
           for (int l = 0; l < 2; ++l) {
-            P[k][l] = __ldg(src_p + (k * RPR * C + l * kPairW));
-            V[k][l] = __ldg(src_v + (k * RPR * C + l * kPairW));
+            P[k][l] = src_p[k * RPR * C + l * kPairW];
+            V[k][l] = src_v[k * RPR * C + l * kPairW];
           }
     }
 #pragma unroll
@@ -672,12 +672,12 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
     }
     // mass and pin flag of the pair, needed after the gather
     if (in0) {
-      m0 = __ldg(&pos[v0].w);
-      pin0 = __ldg(&vel[v0].w);
+      m0 = pos[v0].w;
+      pin0 = vel[v0].w;
     }
     if (in1) {
-      m1 = __ldg(&pos[v1].w);
-      pin1 = __ldg(&vel[v1].w);
+      m1 = pos[v1].w;
+      pin1 = vel[v1].w;
     }
   } else {
     far = halo_struts(std::true_type{});
@@ -807,7 +807,7 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
 template <int TH>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_CTAS)
     k_step_grid_tiled(int R, int C, TileSplit split, int n_ring, const float* __restrict__ params,
-                      const float4* __restrict__ pos, const float4* __restrict__ vel,
+                      const float4* pos, const float4* vel,
                       const float4* __restrict__ force_in, float4* __restrict__ pos_out,
                       float4* __restrict__ vel_out, const __grid_constant__ StepConsts c) {
   int bx, by;

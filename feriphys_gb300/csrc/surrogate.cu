@@ -116,8 +116,8 @@ __device__ __forceinline__ bool group_wait(uint64_t* bar, uint32_t& phase, int i
 
 __device__ __forceinline__ void vertex_features(const SurCloth& c, int parity, int r, int col, float (&f)[kFeat]) {
   const int R = c.rows, C = c.cols;
-  const float4* __restrict__ P = c.pos[parity];
-  const float4* __restrict__ Vl = c.vel[parity];
+  const float4* P = c.pos[parity];
+  const float4* Vl = c.vel[parity];
   const float4* __restrict__ P0 = c.rest;
   const int i = r * C + col;
   const float4 p = P[i], v = Vl[i], p0 = P0[i];
@@ -184,8 +184,8 @@ __device__ __forceinline__ void store_features_half(const SurCloth& c, int parit
   for (int i = 0; i < NL; ++i) f[i] = 0.0f;
   if (valid) {
     const int R = c.rows, C = c.cols, r = v / C, col = v % C;
-    const float4* __restrict__ P = c.pos[parity];
-    const float4* __restrict__ Vl = c.vel[parity];
+    const float4* P = c.pos[parity];
+    const float4* Vl = c.vel[parity];
     const float4* __restrict__ P0 = c.rest;
     const float4 p = P[v], w0 = Vl[v], p0 = P0[v];
     const float ih = c.inv_h, s = c.sv;
@@ -605,7 +605,7 @@ constexpr uint32_t kCA = 0, kCB = 128, kCW2 = 256, kCW1 = 384, kCW3 = 448, kCB2 
 // [64 h, 64 h + 64) with h = lt / 128 in every epilogue; the threads of h = 0
 // form the loss and dY of their row.
 __global__ void __launch_bounds__(kTrThreads, 1)
-    k_train(const unsigned char* __restrict__ X, const float* __restrict__ T, int n_tiles,
+    k_train(const unsigned char* __restrict__ X, const float* T, int n_tiles,
             const unsigned char* __restrict__ blob, float* __restrict__ partials, float dscale, int* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t bar_w, bar_x, bar_m;
@@ -850,7 +850,7 @@ constexpr int kParamGrid = (kNumParams + 1 + kSumCols - 1) / kSumCols;
 constexpr int kSumMost = 256;  // CTAs whose partials fit (32 KB); launch_train's grid is one per SM
 constexpr int kSumRound = 20;  // loads in flight a thread
 
-__device__ __forceinline__ float partial_sums(const float* __restrict__ partials, int ctas,
+__device__ __forceinline__ float partial_sums(const float* partials, int ctas,
                                               float (&buf)[kSumMost][kSumCols]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q = blockIdx.x * kSumCols + lane;
@@ -863,7 +863,7 @@ __device__ __forceinline__ float partial_sums(const float* __restrict__ partials
 #pragma unroll
       for (int j = 0; j < kSumRound; ++j) {
         const int r = r0 + j * kSumWarps;
-        x[j] = ok && r < n ? __ldg(partials + size_t(c0 + r) * kPartialStride + q) : 0.0f;
+        x[j] = ok && r < n ? partials[size_t(c0 + r) * kPartialStride + q] : 0.0f;
       }
 #pragma unroll
       for (int j = 0; j < kSumRound; ++j) {
@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(kParamBlock)
 }
 
 __global__ void __launch_bounds__(kParamBlock)
-    k_adam(const float* __restrict__ partials, int ctas, float* __restrict__ master, float* __restrict__ m,
+    k_adam(const float* partials, int ctas, float* __restrict__ master, float* __restrict__ m,
            float* __restrict__ v, float lr, float beta1, float beta2, float eps, float c1, float c2,
            unsigned char* __restrict__ blob, float* __restrict__ loss_out, float inv_count) {
   __shared__ float buf[kSumMost][kSumCols];
@@ -1103,8 +1103,8 @@ __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ clot
   const int R = c.rows, C = c.cols, n = R * C;
   const int v = w.y + threadIdx.x;
   const int r = v / C, col = v % C;
-  const float4* __restrict__ P = c.pos[parity];
-  const float4* __restrict__ Vl = c.vel[parity];
+  const float4* P = c.pos[parity];
+  const float4* Vl = c.vel[parity];
   float k[5], L[5];
   bool has[5];
   {
@@ -1161,7 +1161,7 @@ __global__ void __launch_bounds__(128) k_check(const SurCloth* __restrict__ clot
 // run, whatever the number of tiles).
 constexpr int kReduceBlock = 256;
 
-__device__ __forceinline__ float2 cloth_sum(const SurCloth& cl, const float2* __restrict__ tile_out,
+__device__ __forceinline__ float2 cloth_sum(const SurCloth& cl, const float2* tile_out,
                                             float2 (&sh)[kReduceBlock]) {
   float E = 0.0f, S = 0.0f;
   for (int k = threadIdx.x; k < cl.ntiles; k += kReduceBlock) {
@@ -1217,9 +1217,8 @@ __global__ void k_copy_unskipped(const ClothDesc* __restrict__ cloths, int from)
 // two graphs' capture and instantiation, per call, took 190 more).  4,096
 // vertices: 43 and 22 (unchecked 19 and 15).
 __global__ void __launch_bounds__(kReduceBlock)
-    k_verdict(const SurCloth* __restrict__ cloths, const float2* __restrict__ tile_out, float* __restrict__ e_old,
-              double* __restrict__ e_ref, float growth, float abs_margin, float max_strain,
-              int* __restrict__ fail, RolloutCtl* ctl, int step) {
+    k_verdict(const SurCloth* __restrict__ cloths, const float2* tile_out, float* e_old, double* e_ref,
+              float growth, float abs_margin, float max_strain, int* fail, RolloutCtl* ctl, int step) {
   __shared__ float2 sh[kReduceBlock];
   const int c = blockIdx.x;
   chain_wait();
