@@ -233,3 +233,25 @@ def test_checked_steps_launched_ahead(fgb, steps):
             assert np.array_equal(a, b), scale
         counts.append(got[0][0])
     assert len(set(counts)) > 1, counts
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [1, 1638, 1639, 5461, 5462])
+def test_reads_into_pageable_and_pinned_memory(fgb, n, bits):
+    """Rows read into pageable memory (through the mesh's own pinned rows up to
+    64 KB: 1,638 points, or 5,461 positions) and into pinned memory are the
+    same bytes."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    m = fgb.SpringyMesh.new(rng.normal(0, 1, (n, 3)).astype(np.float32), [], 0.01 * n, 1.0, 1.0)
+    m.set_precision(bits)
+    sim = fgb.Simulation.new([m], [])
+    sim.step(2)
+    pinned = lambda k: torch.zeros((n, k), pin_memory=True).numpy()  # noqa: E731
+    for _ in range(2):
+        sim.step(1)
+        assert m.get_points().tobytes() == m.get_points(pinned(10)).tobytes()
+        odd = np.zeros(3 * n + 1, np.float32)[1:].reshape(n, 3)
+        assert m.get_positions(odd).tobytes() == m.get_positions(pinned(3)).tobytes()
+        assert odd.tobytes() == m.get_points()[:, 1:4].tobytes()
