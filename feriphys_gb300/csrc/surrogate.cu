@@ -249,7 +249,7 @@ __device__ __forceinline__ void store_features_half(const SurCloth& c, int parit
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int k = col + e < kFeat ? col + e : 0;
-      x[e] = (valid && col + e < kFeat) ? (f[li + e] - nm.in_mean[k]) * nm.in_inv_std[k] : 0.0f;
+      x[e] = col + e < kFeat ? (f[li + e] - nm.in_mean[k]) * nm.in_inv_std[k] : 0.0f;
     }
     *reinterpret_cast<uint2*>(X + tc::blk_off(kIn, row, col)) = make_uint2(pack_bf2(x[0], x[1]), pack_bf2(x[2], x[3]));
   }
@@ -425,6 +425,22 @@ __device__ __forceinline__ bool stopped(const int* stop) {
 // G groups of 128 * H threads; a group takes one 128-vertex tile at a time,
 // H threads per vertex row (H = 2: each computes half of the row's features
 // and half of its hidden columns, so twice the warps hide the latencies).
+//
+// Bound by latency and by what the groups of an SM take turns at: a tile alone
+// on an SM takes about 6 us, four at a time 10, with the issue slots half
+// used.  So:
+//   * tiles go to the SMs first and to the groups of an SM last, which leaves
+//     a remainder spread over all SMs (262,144 vertices, microseconds a step:
+//     52.9 -> 48.4; 4,096 vertices, one tile an SM instead of four: 14.9 -> 8.2);
+//   * the groups start kGroupLag clocks apart, about the time of one tile's
+//     features, and stay so: one group's feature loads then fall into the
+//     others' GELUs instead of all groups doing the same at a time (48.4 ->
+//     39.0; 2,000 clocks 41.5, 4,000 38.9, but 17.5 against 16.8 at 78,400
+//     vertices).  Only from three tiles an SM on: with two, starting later
+//     costs more than it gives (19,600 vertices: 9.2 us without, 9.6 with).
+//     (Passing a token on from group to group instead: 40.3, or 47.4 every round.)
+constexpr int kGroupLag = 3000;  // at 2 GHz: 1.5 us
+
 template <int G, int H>
 __global__ void __launch_bounds__(128 * G * H, 1)
     k_sur_step(const SurCloth* __restrict__ cloths, const Tile* __restrict__ tiles, int n_tiles, int parity,
@@ -462,12 +478,16 @@ __global__ void __launch_bounds__(128 * G * H, 1)
   chain_wait();
   chain_next();
   if (stopped(stop)) n_tiles = 0;
+  if (n_tiles > 2 * int(gridDim.x)) {  // three groups or more at work on some SMs
+    const long long t0 = clock64();
+    while (clock64() - t0 < g * kGroupLag) __nanosleep(50);
+  }
   const uint32_t tmem = tslot + uint32_t(g * 128);
   const uint32_t lane_off = uint32_t((row >> 5) * 32) << 16;
   unsigned char* act = smem + kBlobSmem + g * 32768;
   const ObsFace* faces = static_cast<const ObsFace*>(cst.obstacle_faces);
   uint32_t phase = 0;
-  for (int t = blockIdx.x * G + g; ok && t < n_tiles; t += gridDim.x * G) {
+  for (int t = g * gridDim.x + blockIdx.x; ok && t < n_tiles; t += gridDim.x * G) {
     const Tile w = tiles[t];
     const SurCloth& c = cloths[w.x];
     const int n = c.rows * c.cols;
@@ -1349,7 +1369,7 @@ cudaError_t sur_step_g(const SurCloth* cloths, const Tile* tiles, int n_tiles, i
   const int smem = kBlobSmem + G * 32768;
   const cudaError_t e = sur_step_attr<G, H>();
   if (e != cudaSuccess) return e;
-  int grid = (n_tiles + G - 1) / G;
+  int grid = n_tiles;
   const int cap = ctas > 0 ? ctas : sm_count();
   if (grid > cap) grid = cap;
   if (grid < 1) return cudaSuccess;

@@ -255,3 +255,37 @@ def test_reads_into_pageable_and_pinned_memory(fgb, n, bits):
         odd = np.zeros(3 * n + 1, np.float32)[1:].reshape(n, 3)
         assert m.get_positions(odd).tobytes() == m.get_positions(pinned(3)).tobytes()
         assert odd.tobytes() == m.get_points()[:, 1:4].tobytes()
+
+
+@pytest.mark.parametrize("rows, cols, cloths", [(64, 64, 5), (64, 64, 10), (64, 64, 20), (61, 67, 21), (9, 9, 160)])
+def test_coarse_step_is_the_same_in_any_company(fgb, rows, cols, cloths):
+    """A coarse step of a cloth gives the same bits alone (a tile an SM) and
+    among copies of itself, where its tiles fall to the second, third and
+    fourth group of an SM, to groups that start late and to later rounds; the
+    last tile of a cloth may be partly empty."""
+    s = 0.02
+    rng = np.random.default_rng(rows + cloths)
+    kick = rng.normal(0, 0.3, (rows * cols, 3)).astype(np.float32)
+
+    def sim_of(k):
+        meshes = []
+        for _ in range(k):
+            m = fgb.Cloth.new(rows, cols, s, (0.0, 0.0, 0.0), 0.01, 500.0 * s, 0.5 * s, 250.0 * s, 0.5 * s, 50.0 * s,
+                              0.5 * s, np.asarray([0], np.uint32)).mesh
+            pts = m.get_points()
+            pts[:, 4:7] = kick
+            m.set_points(pts)
+            meshes.append(m)
+        sim = fgb.Simulation.new(meshes, [])
+        sim.set_config(fgb.Config.make(dt=1.0 / 6000.0, gravity=(0.0, -9.8, 0.0), wind=(1.0, 0.5, 0.2)))
+        return sim, meshes
+
+    sur = fgb.Surrogate.new(3)
+    sur.set_normalization(np.zeros(54), np.ones(54), np.zeros(3), np.full(3, 0.05))
+    one, (alone,) = sim_of(1)
+    many, meshes = sim_of(cloths)
+    assert one.step_surrogate(sur, 10, 3) == 0 and many.step_surrogate(sur, 10, 3) == 0
+    want = alone.get_points()
+    assert np.isfinite(want).all() and not np.array_equal(want[:, 4:7], kick)
+    for m in meshes:
+        assert m.get_points().tobytes() == want.tobytes()
