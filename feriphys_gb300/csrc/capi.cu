@@ -197,6 +197,9 @@ void free_topology(fgb_mesh* m) {
   dfree(m->d_strut_word16);
   dfree(m->d_face_word);
   m->compact_form = 0;
+  dfree(m->d_strut_ab);
+  dfree(m->d_strut_term);
+  dfree(m->d_face_term);
   dfree(m->d_grid);
   dfree(m->d_rest);
   m->csr_ready = false;
@@ -334,6 +337,11 @@ fgb::GeneralTopo general_topo(const fgb_mesh* m) {
     t.strut_word16 = m->d_strut_word16;
     t.face_word = m->d_face_word;
   }
+  t.strut_term = m->d_strut_term;
+  t.face_term = m->d_face_term;
+  t.strut_ab = m->d_strut_ab;
+  t.n_struts = int(m->topo.sa.size());
+  t.n_faces = int(m->topo.fv.size() / 3);
   return t;
 }
 
@@ -343,6 +351,24 @@ int decide_path(fgb_mesh* m, int* path) {
   if (m->path_req == 2 && !grid_ok)
     return fail(FGB_ESTATE, "grid path requested but the mesh is not a Cloth::new grid (or precision is f64)");
   *path = (m->path_req == 1 || !grid_ok) ? 1 : 2;
+  return FGB_OK;
+}
+
+// The FP64 step's scratch and the struts' points; without room for them the
+// step does without.
+int ensure_terms64(fgb_mesh* m) {
+  const size_t faces = m->topo.fv.size() / 3, struts = m->topo.sa.size();
+  if (dalloc(m->d_strut_term, 48 * struts) != cudaSuccess || dalloc(m->d_face_term, 48 * faces) != cudaSuccess ||
+      dalloc(m->d_strut_ab, sizeof(int2) * struts) != cudaSuccess) {
+    cudaGetLastError();
+    dfree(m->d_strut_term);
+    dfree(m->d_face_term);
+    dfree(m->d_strut_ab);
+    return FGB_OK;
+  }
+  std::vector<int2> ab(struts);
+  for (size_t i = 0; i < struts; ++i) ab[i] = make_int2(int(m->topo.sa[i]), int(m->topo.sb[i]));
+  FGB_CUDA(cudaMemcpy(m->d_strut_ab, ab.data(), sizeof(int2) * struts, cudaMemcpyHostToDevice));
   return FGB_OK;
 }
 
@@ -358,6 +384,7 @@ int ensure_topology(fgb_mesh* m) {
     FGB_CUDA(cudaMemcpy(m->d_grid, params.data(), params.size() * sizeof(float), cudaMemcpyHostToDevice));
   } else {
     FGB_CHECK_RC(ensure_csr(m));
+    if (m->precision == 64) FGB_CHECK_RC(ensure_terms64(m));
   }
   m->topo_dirty = false;
   return FGB_OK;

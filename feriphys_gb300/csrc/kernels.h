@@ -27,6 +27,12 @@ struct GeneralTopo {
   const uint32_t* strut_word = nullptr;
   const uint16_t* strut_word16 = nullptr;
   const uint16_t* face_word = nullptr;
+  // FP64 scratch: 6 doubles a strut (spring, damper) and a face (force, three
+  // corner weights); null: the step evaluates them vertex by vertex
+  double* strut_term = nullptr;
+  double* face_term = nullptr;
+  const int2* strut_ab = nullptr;  // with them: the struts' points
+  int n_struts = 0, n_faces = 0;
 };
 
 // Grid (Cloth::new topology) description for the stencil kernel (see

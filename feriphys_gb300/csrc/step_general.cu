@@ -146,10 +146,10 @@ __device__ __forceinline__ void flag_nonfinite(bool bad, unsigned* flags) {
 // Fused Simulation::step for one mesh (accumulate -> integrate -> collide ->
 // pin restore -> clear), one thread per vertex.  The f32 form asks for 4
 // blocks of 256 per SM (at most 64 registers: the gather is latency-bound, so
-// resident warps count); the FP64 rerun, bound by the FP64 units (one warp
-// instruction takes one of them 64 cycles), takes single-warp blocks so that a
-// mesh reaches as many of them as it has warps (90 x 61 tube: 123 us a step
-// with blocks of 256, 64 with 32).
+// resident warps count).  FP64 comes here only without room for k_terms64's
+// scratch; bound by the FP64 units (one warp instruction takes one of them 64
+// cycles), it takes single-warp blocks so that a mesh reaches as many of them
+// as it has warps (90 x 61 tube: 123 us a step with blocks of 256, 64 with 32).
 template <class T> constexpr int kStepBlock = sizeof(T) == 4 ? 256 : 32;
 template <class T, int FORM>
 __global__ void __launch_bounds__(kStepBlock<T>, sizeof(T) == 4 ? 4 : 1)
@@ -191,16 +191,15 @@ __global__ void __launch_bounds__(kStepBlock<T>, sizeof(T) == 4 ? 4 : 1)
 // warp 0 adds those in face order, integrates and collides.  The same terms in
 // the same order, so the same bits as k_step_general; a vertex's chain of
 // terms is what a step of a small or slow mesh waits for (see the launch).
-template <class T> struct SplitShape;
-template <> struct SplitShape<float> { static constexpr int NF = 3, PER = 2; };
-template <> struct SplitShape<double> { static constexpr int NF = 6, PER = 1; };
+constexpr int kSplitFaceWarps = 3, kSplitFacesEach = 2;
 
-template <class T, int FORM>
-__global__ void __launch_bounds__(32 * (SplitShape<T>::NF + 1))
-    k_step_split(int n, const Vec4<T>* pos, const Vec4<T>* vel,
-                 const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
+template <int FORM>
+__global__ void __launch_bounds__(32 * (kSplitFaceWarps + 1))
+    k_step_split(int n, const float4* pos, const float4* vel, const float4* __restrict__ force_in,
+                 float4* __restrict__ pos_out, float4* __restrict__ vel_out,
                  GeneralTopo t, StepConsts c) {
-  constexpr int NF = SplitShape<T>::NF, PER = SplitShape<T>::PER, SLOTS = NF * PER;
+  using T = float;
+  constexpr int NF = kSplitFaceWarps, SLOTS = NF * kSplitFacesEach;
   __shared__ T share[SLOTS][3][32];
   __shared__ int s_rounds;
   const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
@@ -264,6 +263,124 @@ __global__ void __launch_bounds__(32 * (SplitShape<T>::NF + 1))
   pos_out[v] = make4<T>(np, m);
   vel_out[v] = make4<T>(nv, V4.w);
   flag_nonfinite(!(finite3(np) && finite3(nv)), c.flags);
+}
+
+// FP64 in two launches: every strut's and every face's terms once
+// (k_terms64), then per vertex their sum in the same order, the integration
+// and the collisions (k_gather64).  The same values, so the same bits as
+// k_step_general, which evaluates a strut twice, a face's force three times
+// and its cross product six times: the FP64 units bound this step (see
+// kStepBlock), and the terms' 96 bytes a strut and face written and read cost
+// little beside them.  Blocks of the terms are single warps, the long ones
+// first, so that a small mesh reaches every unit.  A face has four threads
+// (its force, and each corner's share, which needs the cross product again) up
+// to kWholeFaces and one beyond, where the units are full anyway (us a step,
+// four and one: 10,800 faces 17.5 and 18.4, 42,000 40 and 67, 60,000 59 and
+// 60, 120,000 104 and 94, 240,000 197 and 168).
+constexpr int kWholeFaces = 65536;
+
+template <int ROLES>
+__global__ void __launch_bounds__(32) k_terms64(const Dbl4* pos, const Dbl4* vel, GeneralTopo t, StepConsts c) {
+  const int nbf = (t.n_faces + 31) / 32, role = nbf > 0 ? min(int(blockIdx.x) / nbf, ROLES) : ROLES;
+  if (role < ROLES) {
+    const int f = (int(blockIdx.x) - role * nbf) * 32 + int(threadIdx.x);
+    const int4 w = t.face_vtx[min(f, t.n_faces - 1)];
+    chain_wait();
+    chain_next();
+    if (f >= t.n_faces) return;
+    const V3<double> x0 = xyz<double>(pos[w.x]), x1 = xyz<double>(pos[w.y]), x2 = xyz<double>(pos[w.z]);
+    double* out = t.face_term + 6 * size_t(f);
+    if (ROLES == 1)
+      for (int k = 0; k < 3; ++k) out[3 + k] = face_corner_weight<double>(x0, x1, x2, k);
+    else if (role < 3)
+      out[3 + role] = face_corner_weight<double>(x0, x1, x2, role);
+    if (role == ROLES - 1) {
+      const V3<double> D = face_total_force<double>(
+          x0, x1, x2, xyz<double>(vel[w.x]), xyz<double>(vel[w.y]), xyz<double>(vel[w.z]),
+          V3<double>{double(c.wind[0]), double(c.wind[1]), double(c.wind[2])}, double(c.neg_drag), double(c.neg_lift));
+      out[0] = D.x;
+      out[1] = D.y;
+      out[2] = D.z;
+    }
+    return;
+  }
+  const int e = (int(blockIdx.x) - ROLES * nbf) * 32 + int(threadIdx.x);
+  const int2 ab = t.strut_ab[min(e, t.n_struts - 1)];
+  const float4 kcl = t.strut_kcl[min(e, t.n_struts - 1)];
+  chain_wait();
+  chain_next();
+  if (e >= t.n_struts) return;
+  V3<double> sf, df;
+  strut_forces<double>(xyz<double>(pos[ab.x]), xyz<double>(pos[ab.y]), xyz<double>(vel[ab.x]), xyz<double>(vel[ab.y]),
+                       double(kcl.x), double(kcl.y), double(kcl.z), sf, df);
+  double2* out = reinterpret_cast<double2*>(t.strut_term + 6 * size_t(e));
+  out[0] = make_double2(sf.x, sf.y);
+  out[1] = make_double2(sf.z, df.x);
+  out[2] = make_double2(df.y, df.z);
+}
+
+// The sums and the integration are the same for each component, so a vertex
+// has three threads, in three warps; only the collisions, where there are
+// obstacles, take one.
+__global__ void __launch_bounds__(96) k_gather64(int n, const double* pos, const double* vel, const double* force_in,
+                                                 double* pos_out, double* vel_out, GeneralTopo t, StepConsts c) {
+  __shared__ double sh[9][32];
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  const int v = blockIdx.x * 32 + lane;
+  const bool vertex = v < n;
+  const int s_beg = vertex ? t.strut_off[v] : 0, s_end = vertex ? t.strut_off[v + 1] : 0;
+  const int f_beg = vertex ? t.face_off[v] : 0, f_end = vertex ? t.face_off[v + 1] : 0;
+  chain_wait();
+  chain_next();
+  const size_t at = 4 * size_t(vertex ? v : 0);
+  const double m = pos[at + 3], pin = vel[at + 3], p = pos[at + k], w = vel[at + k];
+  const bool free = vertex && pin == 0.0;  // pinned: update_points restores the old point (springy_mesh.rs:492-496)
+  double F = double(c.force0[k]);
+  if (force_in) F = force_in[at + k] + F;
+  if (free) {
+#pragma unroll 2
+    for (int e = s_beg; e < s_end; ++e) {
+      const int s = t.strut_inc[e].y;
+      const double* q = t.strut_term + 6 * size_t(s >> 1) + k;
+      const long long sign = (long long)(s & 1) << 63;  // the second point's: times -1
+      F = F + __longlong_as_double(__double_as_longlong(q[0]) ^ sign);
+      F = F + __longlong_as_double(__double_as_longlong(q[3]) ^ sign);
+    }
+#pragma unroll 2
+    for (int e = f_beg; e < f_end; ++e) {
+      const int f = t.face_inc[e];
+      const double* q = t.face_term + 6 * size_t(f >> 2);
+      F = F + q[3 + (f & 3)] * q[k];
+    }
+  }
+  V3<double> np, nv, nF;
+  integrate_point<double>(c.integration, double(c.dt), V3<double>{p, 0.0, 0.0}, V3<double>{w, 0.0, 0.0},
+                          V3<double>{F, 0.0, 0.0}, m, np, nv, nF);
+  if (c.n_obstacle_faces > 0) {
+    sh[k][lane] = F;
+    sh[3 + k][lane] = np.x;
+    sh[6 + k][lane] = nv.x;
+    __syncthreads();
+    if (k == 0 && free) {
+      const V3<double> P{p, pos[at + 1], pos[at + 2]}, V{w, vel[at + 1], vel[at + 2]};
+      V3<double> n3{sh[3][lane], sh[4][lane], sh[5][lane]}, v3{sh[6][lane], sh[7][lane], sh[8][lane]};
+      collide_point<double>(static_cast<const ObsFace*>(c.obstacle_faces), c.n_obstacle_faces, P, V,
+                            V3<double>{sh[0][lane], sh[1][lane], sh[2][lane]}, m, n3, v3, c);
+      sh[3][lane] = n3.x; sh[4][lane] = n3.y; sh[5][lane] = n3.z;
+      sh[6][lane] = v3.x; sh[7][lane] = v3.y; sh[8][lane] = v3.z;
+    }
+    __syncthreads();
+    np.x = sh[3 + k][lane];
+    nv.x = sh[6 + k][lane];
+  }
+  if (!vertex) return;
+  pos_out[at + k] = free ? np.x : p;
+  vel_out[at + k] = free ? nv.x : w;
+  if (k == 0) {
+    pos_out[at + 3] = m;
+    vel_out[at + 3] = pin;
+  }
+  if (free) flag_nonfinite(!(isfinite(np.x) && isfinite(nv.x)), c.flags);
 }
 
 // accumulate_forces: force[v] = force[v] + gravity + struts + faces; pins -> 0.
@@ -337,19 +454,37 @@ cudaError_t launch_step_general(int n, const void* pos, const void* vel, const v
                  static_cast<const Vec4<T>*>(vel), static_cast<const Vec4<T>*>(force_in),
                  static_cast<Vec4<T>*>(pos_out), static_cast<Vec4<T>*>(vel_out), t, c);
   };
-  // Up to this many vertices a step takes as long as one vertex's chain of
-  // terms, which the split kernel shortens; beyond, the SMs are full and its
-  // shared-memory exchange only costs (tubes, us a step, one thread per vertex
-  // against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3, 360 x 280 14.4
-  // -> 18.6; FP64, before its terms were fused, 12 x 10 64 -> 29, 90 x 61 64
-  // -> 39, 300 x 200 207 -> 220).
+  if constexpr (sizeof(T) == 8) {
+    // (90 x 61 tube: 29.4 us a step in one launch, 17.5 in two; 12 x 10: 24 and 12; 300 x 200: 161 and 94)
+    if (t.strut_term && t.face_term) {
+      const bool whole = t.n_faces > kWholeFaces;
+      const int terms = (whole ? 1 : 4) * blocks_for(t.n_faces, 32) + blocks_for(t.n_struts, 32);
+      if (terms > 0) {
+        const cudaError_t e = chain_launch(whole ? k_terms64<1> : k_terms64<4>, terms, 32, 0, s, chained, static_cast<const Dbl4*>(pos),
+                                           static_cast<const Dbl4*>(vel), t, c);
+        if (e != cudaSuccess) return e;
+      }
+      return chain_launch(k_gather64, blocks_for(n, 32), 96, 0, s, chained || terms > 0, n,
+                          static_cast<const double*>(pos), static_cast<const double*>(vel),
+                          static_cast<const double*>(force_in), static_cast<double*>(pos_out),
+                          static_cast<double*>(vel_out), t, c);
+    }
+  }
+  // f32: up to this many vertices a step takes as long as one vertex's chain
+  // of terms, which the split kernel shortens; beyond, the SMs are full and
+  // its shared-memory exchange only costs (tubes, us a step, one thread per
+  // vertex against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3,
+  // 360 x 280 14.4 -> 18.6).
   constexpr int kSplitMost = 32768;
-  if (n <= kSplitMost)
-    run(t.form == 2 ? k_step_split<T, 2> : (t.form == 1 ? k_step_split<T, 1> : k_step_split<T, 0>),
-        blocks_for(n, 32), 32 * (SplitShape<T>::NF + 1));
-  else
-    run(t.form == 2 ? k_step_general<T, 2> : (t.form == 1 ? k_step_general<T, 1> : k_step_general<T, 0>),
-        blocks_for(n, kStepBlock<T>), kStepBlock<T>);
+  if constexpr (sizeof(T) == 4) {
+    if (n <= kSplitMost) {
+      run(t.form == 2 ? k_step_split<2> : (t.form == 1 ? k_step_split<1> : k_step_split<0>), blocks_for(n, 32),
+          32 * (kSplitFaceWarps + 1));
+      return cudaGetLastError();
+    }
+  }
+  run(t.form == 2 ? k_step_general<T, 2> : (t.form == 1 ? k_step_general<T, 1> : k_step_general<T, 0>),
+      blocks_for(n, kStepBlock<T>), kStepBlock<T>);
   return cudaGetLastError();
 }
 

@@ -289,3 +289,51 @@ def test_coarse_step_is_the_same_in_any_company(fgb, rows, cols, cloths):
     assert np.isfinite(want).all() and not np.array_equal(want[:, 4:7], kick)
     for m in meshes:
         assert m.get_points().tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("integration", [0, 1])
+@pytest.mark.parametrize("rows, cols, faces", [(1, 2, True), (2, 2, True), (5, 7, True), (9, 9, False), (33, 31, True),
+                                               (190, 180, True)])
+def test_f64_step_is_its_phases(fgb, rows, cols, faces, integration):
+    """The FP64 step (terms once each, then per vertex) gives the bits of its
+    phases called one by one (accumulate_forces sums vertex by vertex), for
+    loose points, few and many faces, struts without faces, pins, carried
+    forces and an obstacle."""
+    from feriphys_gb300 import workloads as W
+
+    rng = np.random.default_rng(rows + 10 * cols)
+    y, x = np.mgrid[0:rows, 0:cols]
+    pos = np.stack([x * 0.1, 0.02 * rng.normal(0, 1, x.shape), y * 0.1], -1).reshape(-1, 3).astype(np.float32)
+    v = np.arange(rows * cols).reshape(rows, cols)
+    a, b, c, d = (q.reshape(-1) for q in (v[:-1, :-1], v[:-1, 1:], v[1:, :-1], v[1:, 1:]))
+    idx = np.stack([a, b, c, b, d, c], 1).reshape(-1).astype(np.uint32) if faces else np.zeros(0, np.uint32)
+    cfg = fgb.Config.make(integration=integration, dt=1.0 / 2000.0, gravity=(0.0, -0.1, 0.0), wind=(2.0, 0.5, 1.0),
+                          lift_coefficient=0.3, drag_coefficient=0.6, coefficient_of_restitution=0.3,
+                          coefficient_of_friction=0.2)
+    obstacle = fgb.CollidableMesh.new(*W.plane(-0.03, 40.0))
+    state = None
+    out = []
+    for whole in (True, False):
+        m = fgb.SpringyMesh.new(pos, idx, 0.01 * len(pos), 5.0, 0.01)
+        if not faces:
+            m.add_struts(np.stack([v[:, :-1].reshape(-1), v[:, 1:].reshape(-1)], 1)[::2], 4.0, 0.02)
+        m.add_pins([0])
+        m.set_precision(64)
+        sim = fgb.Simulation.new([m], [obstacle])
+        sim.set_config(cfg)
+        sim.step(0)
+        if state is None:
+            state = m.get_points()
+            state[:, 4:7] = rng.normal(0, 1.0, (len(pos), 3))
+            state[:, 7:10] = rng.normal(0, 0.01, (len(pos), 3))
+        m.set_points(state)
+        for _ in range(4):
+            if whole:
+                sim.step(1)
+            else:
+                m.accumulate_forces(cfg)
+                m.integrate(integration, 1.0 / 2000.0)
+                m.update_points([obstacle], cfg)
+                m.clear_forces()
+        out.append(m.get_points_f64())
+    assert np.isfinite(out[0]).all() and out[0].tobytes() == out[1].tobytes()
