@@ -281,7 +281,7 @@ def run_reference(args, rank, world):
 
 
 def kernels_per_step(mesh, args):
-    """Launches of this library's kernels per step (every step form is one)."""
+    """Launches of this library's kernels per step (every f32 step form is one)."""
     return 1
 
 
@@ -352,7 +352,7 @@ def run_batched(args, rank, world, dist, torch, fgb, W, emit=True):
                                    "per-cloth wind, plane; dt=1/600 Euler; %d-step rollouts as one CUDA graph"
                                    % (len(meshes), n_vert, S, rollout),
                        "l2": "working set (%.1f GB) larger than L2, not flushed" % (B * n_vert / 1e9),
-                       "launch": {"cloths": info[0], "tiles": info[1], "mode": ["per-tile CTAs", "persistent"][info[2]],
+                       "launch": {"cloths": info[0], "tiles": info[1], "mode": "per-tile CTAs",
                                   "ctas": info[3], "tile": "32x%d" % info[4], "chosen_by": "autotuner"}},
             "simulated_seconds_per_s": world * dt / (ms * 1e-3),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

@@ -380,7 +380,7 @@ class SpringyMesh:
         _check(_lib().fgb_mesh_set_strut_params(self._h, _ptr(k), _ptr(c)))
 
     def set_path(self, path: int):
-        """0 auto, 1 general gather, 2 grid (32x8 tiles), 3 grid (one thread per vertex),
+        """0 auto, 1 general gather, 2 grid (tiles), 3 grid (one thread per vertex),
         4 general gather over the plain incidence lists."""
         _check(_lib().fgb_mesh_set_path(self._h, int(path)))
 
@@ -509,7 +509,7 @@ class Simulation:
         return self.get_timestep()
 
     def set_batch_mode(self, mode: int):
-        """-1 autotuned (default), 0 one CTA per tile, 1 persistent."""
+        """-1 (default), 0 or 1: accepted and reported; all run one CTA per tile."""
         _check(_lib().fgb_sim_set_batch_mode(self._h, int(mode)))
 
     def set_batch_tile(self, tile_rows: int):
@@ -520,7 +520,7 @@ class Simulation:
         _check(_lib().fgb_sim_set_graphs(self._h, 1 if enabled else 0))
 
     def batch_info(self):
-        """(meshes in the batch, work items, launch form, persistent CTAs, tile rows)."""
+        """(meshes in the batch, work items, launch form as set, CTAs resident at a time, tile rows)."""
         out = np.zeros(5, np.int64)
         _check(_lib().fgb_sim_batch_info(self._h, _ptr(out)))
         return tuple(int(v) for v in out)

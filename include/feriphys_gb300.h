@@ -229,16 +229,16 @@ int fgb_sim_step(fgb_sim* s, uint64_t n_steps);
 int fgb_mesh_set_wind(fgb_mesh* m, const float* wind);
 
 /* Batched stepping: a simulation with two or more Cloth::new grid meshes
- * advances all of them with one kernel launch per step (largest cloths
- * first, tiles pulled from a shared work list); a call with n_steps >= 2 is
+ * advances all of them with one kernel launch per step (a block per tile of
+ * a shared work list, largest cloths first); a call with n_steps >= 2 is
  * captured once as a CUDA graph and replayed (1 = default; 0 = plain
  * launches).  Extension with no reference counterpart (the reference steps
  * meshes one after another, springy/simulation.rs:28); results are
  * identical to stepping each mesh alone. */
 int fgb_sim_set_graphs(fgb_sim* s, int enabled);
 
-/* Launch form of the batched step: -1 (default) lets the autotuner choose,
- * 0 one CTA per tile, 1 persistent CTAs pulling tiles from a work counter. */
+/* Launch form of the batched step: -1 (default), 0 or 1.  Accepted and
+ * reported; there is one form left, a CTA per tile, which all three run. */
 int fgb_sim_set_batch_mode(fgb_sim* s, int mode);
 
 /* Tile of the batched step: 32 vertices wide and tile_rows = 4, 8 or 12
@@ -248,8 +248,8 @@ int fgb_sim_set_batch_mode(fgb_sim* s, int mode);
 int fgb_sim_set_batch_tile(fgb_sim* s, int tile_rows);
 
 /* out[0] meshes in the batch, out[1] work items (tiles), out[2] launch form
- * chosen by the autotuner (0 one CTA per tile, 1 persistent; -1 not yet
- * tuned), out[3] persistent CTAs, out[4] tile rows.  The choice is cached
+ * (as set, 0 by default; -1 before the batch is tuned), out[3] CTAs the GPU
+ * holds at a time, out[4] tile rows.  The autotuner's tile is cached
  * per GPU in $FGB_AUTOTUNE_CACHE (default ~/.cache/feriphys_gb300/autotune.txt). */
 int fgb_sim_batch_info(const fgb_sim* s, int64_t out[5]);
 
@@ -270,8 +270,8 @@ int fgb_sim_set_stream(fgb_sim* s, void* stream);
  * engines and renderers that own all GPU memory through their own
  * allocators, and real-time loops that cannot afford cudaMalloc/cudaFree,
  * which may synchronise the whole device.  Advances every mesh of a
- * simulation n_steps times with the batched persistent kernel, keeping its
- * scratch (work counter, cloth table, tile list) in a fixed 4 MiB array that
+ * simulation n_steps times with the batched kernel, keeping its
+ * scratch (cloth table, tile list) in a fixed 4 MiB array that
  * every GPU loading this library holds until exit: it fits 80 bytes per cloth
  * plus 16 bytes per 32x8 tile (e.g. 4096 cloths of 16..128 vertices a side
  * need 2.3 MB); larger batches fail with FGB_EINVAL.  Inputs
