@@ -359,16 +359,15 @@ int decide_path(fgb_mesh* m, int* path) {
 int ensure_terms64(fgb_mesh* m) {
   const size_t faces = m->topo.fv.size() / 3, struts = m->topo.sa.size();
   if (dalloc(m->d_strut_term, 48 * struts) != cudaSuccess || dalloc(m->d_face_term, 48 * faces) != cudaSuccess ||
-      dalloc(m->d_strut_ab, sizeof(int2) * struts) != cudaSuccess) {
+      dalloc(m->d_strut_ab, 2 * sizeof(uint32_t) * struts) != cudaSuccess) {
     cudaGetLastError();
     dfree(m->d_strut_term);
     dfree(m->d_face_term);
     dfree(m->d_strut_ab);
     return FGB_OK;
   }
-  std::vector<int2> ab(struts);
-  for (size_t i = 0; i < struts; ++i) ab[i] = make_int2(int(m->topo.sa[i]), int(m->topo.sb[i]));
-  FGB_CUDA(cudaMemcpy(m->d_strut_ab, ab.data(), sizeof(int2) * struts, cudaMemcpyHostToDevice));
+  FGB_CUDA(cudaMemcpy(m->d_strut_ab, m->topo.sa.data(), sizeof(uint32_t) * struts, cudaMemcpyHostToDevice));
+  FGB_CUDA(cudaMemcpy(m->d_strut_ab + struts, m->topo.sb.data(), sizeof(uint32_t) * struts, cudaMemcpyHostToDevice));
   return FGB_OK;
 }
 

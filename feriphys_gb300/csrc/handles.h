@@ -89,7 +89,7 @@ struct fgb_mesh {
   uint16_t* d_strut_word16 = nullptr;
   uint16_t* d_face_word = nullptr;
   int compact_form = 0;  // 0 none, 1 32-bit strut words, 2 16-bit strut words
-  int2* d_strut_ab = nullptr;
+  uint32_t* d_strut_ab = nullptr;
   double *d_strut_term = nullptr, *d_face_term = nullptr;  // FP64 step scratch (kernels.h: GeneralTopo)
   // grid topology
   float* d_grid = nullptr;

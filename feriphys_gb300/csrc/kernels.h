@@ -31,7 +31,7 @@ struct GeneralTopo {
   // corner weights); null: the step evaluates them vertex by vertex
   double* strut_term = nullptr;
   double* face_term = nullptr;
-  const int2* strut_ab = nullptr;  // with them: the struts' points
+  const uint32_t* strut_ab = nullptr;  // with them: the struts' first points, then their second ones
   int n_struts = 0, n_faces = 0;
 };
 

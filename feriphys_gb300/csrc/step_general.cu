@@ -305,13 +305,14 @@ __global__ void __launch_bounds__(32) k_terms64(const Dbl4* pos, const Dbl4* vel
     return;
   }
   const int e = (int(blockIdx.x) - ROLES * nbf) * 32 + int(threadIdx.x);
-  const int2 ab = t.strut_ab[min(e, t.n_struts - 1)];
-  const float4 kcl = t.strut_kcl[min(e, t.n_struts - 1)];
+  const int i = min(e, t.n_struts - 1);
+  const uint32_t a = t.strut_ab[i], b = t.strut_ab[t.n_struts + i];
+  const float4 kcl = t.strut_kcl[i];
   chain_wait();
   chain_next();
   if (e >= t.n_struts) return;
   V3<double> sf, df;
-  strut_forces<double>(xyz<double>(pos[ab.x]), xyz<double>(pos[ab.y]), xyz<double>(vel[ab.x]), xyz<double>(vel[ab.y]),
+  strut_forces<double>(xyz<double>(pos[a]), xyz<double>(pos[b]), xyz<double>(vel[a]), xyz<double>(vel[b]),
                        double(kcl.x), double(kcl.y), double(kcl.z), sf, df);
   double2* out = reinterpret_cast<double2*>(t.strut_term + 6 * size_t(e));
   out[0] = make_double2(sf.x, sf.y);
@@ -474,7 +475,7 @@ cudaError_t launch_step_general(int n, const void* pos, const void* vel, const v
   // of terms, which the split kernel shortens; beyond, the SMs are full and
   // its shared-memory exchange only costs (tubes, us a step, one thread per
   // vertex against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3,
-  // 360 x 280 14.4 -> 18.6).
+  // 360 x 280 14.4 -> 18.6; with launches chained 6.2, 6.4 and, unsplit, 13.9).
   constexpr int kSplitMost = 32768;
   if constexpr (sizeof(T) == 4) {
     if (n <= kSplitMost) {

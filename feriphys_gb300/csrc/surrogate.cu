@@ -1234,8 +1234,10 @@ __global__ void k_copy_unskipped(const ClothDesc* __restrict__ cloths, int from)
 // 83 as a graph of step, check, reduction, decision, and a conditional node
 // with the fallback; 76 with one verdict kernel and chained launches in it;
 // 63 launched ahead without a graph (the conditional node alone is 11; the
-// two graphs' capture and instantiation, per call, took 190 more).  4,096
-// vertices: 43 and 22 (unchecked 19 and 15).
+// two graphs' capture and instantiation, per call, took 190 more); 52 now that
+// the step takes 39.  4,096 vertices: 43, then 22 (unchecked 19 and 15), 15
+// now (8).  (Judged by the check's last block instead of a kernel of its own:
+// 54 and 14.5.)
 __global__ void __launch_bounds__(kReduceBlock)
     k_verdict(const SurCloth* __restrict__ cloths, const float2* tile_out, float* e_old, double* e_ref,
               float growth, float abs_margin, float max_strain, int* fail, RolloutCtl* ctl, int step) {
