@@ -1384,8 +1384,6 @@ cudaError_t sur_step_g(const SurCloth* cloths, const Tile* tiles, int n_tiles, i
 // Threads per vertex row in k_sur_step.
 constexpr int kRowThreads = 2;
 
-int sur_step_max_ctas(int) { return sm_count(); }
-
 cudaError_t launch_sur_step(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, const void* blob,
                             const Norm& norm, const StepConsts& consts, int groups, int ctas, int* err,
                             cudaStream_t s, bool chained, const int* stop) {

@@ -96,7 +96,6 @@ using Tile = int2;
 cudaError_t launch_sur_step(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, const void* blob,
                             const Norm& norm, const StepConsts& consts, int groups, int ctas, int* err,
                             cudaStream_t s, bool chained, const int* stop = nullptr);
-int sur_step_max_ctas(int groups);
 
 // Network outputs (standardised units, bias included) for standardised
 // inputs X (bf16, blocked layout, n_rows a multiple of 128): Y[n][4].
