@@ -53,10 +53,11 @@ template <class T> __device__ __forceinline__ V3<T> cross(V3<T> a, V3<T> b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 #if defined(__CUDACC__)
-// The same with the second product fused (one rounding less each): the face
-// terms of both precisions, and everything of the FP64 rerun -- its error is
-// far below what it is used to state, and the FP64 units bound it (300 x 200
-// tube 207 -> 144 us a step).
+// The same with the second product fused (one rounding less each), for the
+// face terms of both precisions and the struts of the FP64 rerun, by name only:
+// the collision search decides by the sign of a difference of products, which
+// is zero for a point on a face's edge only while both are rounded, and a point
+// on the edge two faces share then counts as inside (tests/test_gpu_collision_f64.py).
 __device__ __forceinline__ float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fused(double a, double b, double c) { return fma(a, b, c); }
 template <class T> __device__ __forceinline__ T fdot(V3<T> a, V3<T> b) {
@@ -65,8 +66,9 @@ template <class T> __device__ __forceinline__ T fdot(V3<T> a, V3<T> b) {
 template <class T> __device__ __forceinline__ V3<T> fcross(V3<T> a, V3<T> b) {
   return {fused(a.y, b.z, -(a.z * b.y)), fused(a.z, b.x, -(a.x * b.z)), fused(a.x, b.y, -(a.y * b.x))};
 }
-__device__ __forceinline__ double dot(V3<double> a, V3<double> b) { return fdot(a, b); }
-__device__ __forceinline__ V3<double> cross(V3<double> a, V3<double> b) { return fcross(a, b); }
+// The struts' dot product: the reference's in f32, fused in the FP64 rerun.
+__device__ __forceinline__ float strut_dot(V3<float> a, V3<float> b) { return dot(a, b); }
+__device__ __forceinline__ double strut_dot(V3<double> a, V3<double> b) { return fdot(a, b); }
 #endif
 __device__ __forceinline__ float sq_root(float v) { return sqrtf(v); }
 __device__ __forceinline__ double sq_root(double v) { return sqrt(v); }

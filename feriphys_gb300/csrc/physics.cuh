@@ -21,9 +21,10 @@ template <class T>
 __device__ __forceinline__ void strut_forces(V3<T> p0, V3<T> p1, V3<T> v0, V3<T> v1, T k, T c, T L, V3<T>& sf,
                                              V3<T>& df) {
   const V3<T> d = p1 - p0;
-  const V3<T> u = normalize(d);
-  sf = (k * (magnitude(d) - L)) * u;
-  df = (c * dot(v1 - v0, u)) * u;
+  const T len = sq_root(strut_dot(d, d));
+  const V3<T> u = d * inv_magnitude(len);
+  sf = (k * (len - L)) * u;
+  df = (c * strut_dot(v1 - v0, u)) * u;
 }
 
 // drag + lift of one face (springy_mesh.rs:634-646): with the face's area A,
