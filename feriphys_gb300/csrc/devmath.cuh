@@ -53,22 +53,41 @@ template <class T> __device__ __forceinline__ V3<T> cross(V3<T> a, V3<T> b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 #if defined(__CUDACC__)
-// The same with the second product fused (one rounding less each), for the
-// face terms of both precisions and the struts of the FP64 rerun, by name only:
-// the collision search decides by the sign of a difference of products, which
-// is zero for a point on a face's edge only while both are rounded, and a point
-// on the edge two faces share then counts as inside (tests/test_gpu_collision_f64.py).
+// The same with the second product fused (one rounding less each), by name only:
+// dot products of the face terms of both precisions, and what the FP64 rerun
+// computes of struts and faces, whose units bound it.  Where a difference of two
+// equal products has to be exactly zero it stays as above: a point on the edge
+// two faces share counts as inside (tests/test_gpu_collision_f64.py), a face
+// whose corners are collinear has no normal (tests/test_gpu_collinear_faces.py).
 __device__ __forceinline__ float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fused(double a, double b, double c) { return fma(a, b, c); }
 template <class T> __device__ __forceinline__ T fdot(V3<T> a, V3<T> b) {
   return fused(a.z, b.z, fused(a.y, b.y, a.x * b.x));
 }
-template <class T> __device__ __forceinline__ V3<T> fcross(V3<T> a, V3<T> b) {
-  return {fused(a.y, b.z, -(a.z * b.y)), fused(a.z, b.x, -(a.x * b.z)), fused(a.x, b.y, -(a.y * b.x))};
-}
-// The struts' dot product: the reference's in f32, fused in the FP64 rerun.
+// Struts' dot product and a face's cross products: the reference's rounding in
+// f32, fused in FP64.
 __device__ __forceinline__ float strut_dot(V3<float> a, V3<float> b) { return dot(a, b); }
 __device__ __forceinline__ double strut_dot(V3<double> a, V3<double> b) { return fdot(a, b); }
+__device__ __forceinline__ V3<float> face_cross(V3<float> a, V3<float> b) { return cross(a, b); }
+__device__ __forceinline__ V3<double> face_cross(V3<double> a, V3<double> b) {
+  return {fused(a.y, b.z, -(a.z * b.y)), fused(a.z, b.x, -(a.x * b.z)), fused(a.x, b.y, -(a.y * b.x))};
+}
+// The cross product a face's normal is made of.  Two products that round to the
+// same p leave at most 2^-53 |p| when fused; only if every component is that
+// small can the unfused one be zero, and then it is taken.  (The test is integer
+// work: with every cross product unfused a 175 x 120 tube takes 42.4 us a step,
+// 40.1 so.)
+__device__ __forceinline__ V3<float> normal_cross(V3<float> a, V3<float> b) { return cross(a, b); }
+__device__ __forceinline__ bool within_rounding(double c, double p) {
+  const int hc = __double2hiint(c) & 0x7fffffff, hp = __double2hiint(p) & 0x7fffffff;
+  return (hc | __double2loint(c)) == 0 || hp < (60 << 20) || hc <= hp - (52 << 20);
+}
+__device__ __forceinline__ V3<double> normal_cross(V3<double> a, V3<double> b) {
+  const V3<double> c = face_cross(a, b);
+  if (within_rounding(c.x, a.z * b.y) && within_rounding(c.y, a.x * b.z) && within_rounding(c.z, a.y * b.x))
+    return cross(a, b);
+  return c;
+}
 #endif
 __device__ __forceinline__ float sq_root(float v) { return sqrtf(v); }
 __device__ __forceinline__ double sq_root(double v) { return sqrt(v); }

@@ -21,15 +21,15 @@ struct FacePair {
 };
 template <bool FAST>
 __device__ __forceinline__ FacePair face_pair(V3x2 x0, V3x2 x1, V3x2 x2, V3x2 v0, V3x2 v1, V3x2 v2, V3x2 nwind,
-                                              f2 neg_cd, f2 neg_lift, uint32_t& far) {
+                                              f2 neg_cd, f2 neg_lift, f2 one, uint32_t& far) {
   const V3x2 sum = add3(add3(v0, v1), v2);
   const f2 r3 = dup2(kRcp3);
   const V3x2 rv{fma2(sum.x, r3, nwind.x), fma2(sum.y, r3, nwind.y), fma2(sum.z, r3, nwind.z)};
   const V3x2 e1 = sub3(x1, x0), e2 = sub3(x2, x0), e3 = sub3(x1, x2);
-  const V3x2 cr = fcross3(e1, sub3(x0, x1), e2);
+  const V3x2 cr = cross3(e1, e2, one);
   f2 mag, inv;
   root_and_rcp<FAST>(fdot3(cr, cr), mag, inv, far);
-  const V3x2 n = scale3(inv, cr), nr = fcross3(n, scale3(mul2(inv, dup2(-1.0f)), cr), rv);
+  const V3x2 n = scale3(inv, cr), nr = cross3(n, rv, one);
   const f2 eff = mul2(mul2(mag, dup2(0.5f)), abs2(fdot3(n, rv)));
   const f2 m2 = root_or_zero<FAST>(fdot3(nr, nr), far);
   return {scale3(mul2(eff, fma2(neg_lift, m2, neg_cd)), rv), mag, fdot3(e2, e1), fdot3(e1, e3)};
@@ -76,11 +76,11 @@ __device__ __forceinline__ void face_terms2(V3x2 x0, V3x2 x1, V3x2 x2, V3x2 v0, 
   const f2 one = dup2(one_rt);
   const V3x2 nwind{neg2(wind.x), neg2(wind.y), neg2(wind.z)};
   uint32_t far = 0;
-  FacePair f[1] = {face_pair<true>(x0, x1, x2, v0, v1, v2, nwind, dup2(neg_cd), dup2(neg_lift), far)};
+  FacePair f[1] = {face_pair<true>(x0, x1, x2, v0, v1, v2, nwind, dup2(neg_cd), dup2(neg_lift), one, far)};
   f2 w0[1], w1[1];
   face_shares<true>(f, one, w0, w1, far);
   if (far > kRootSpan) {
-    f[0] = face_pair<false>(x0, x1, x2, v0, v1, v2, nwind, dup2(neg_cd), dup2(neg_lift), far);
+    f[0] = face_pair<false>(x0, x1, x2, v0, v1, v2, nwind, dup2(neg_cd), dup2(neg_lift), one, far);
     face_shares<false>(f, one, w0, w1, far);
   }
   const float2 dx = upk(f[0].D.x), dy = upk(f[0].D.y), dz = upk(f[0].D.z), u0 = upk(w0[0]), u1 = upk(w1[0]),

@@ -32,11 +32,11 @@ __device__ __forceinline__ V3x2 add_p3(V3x2 F, V3x2 p, f2 one) {
 __device__ __forceinline__ f2 dot3(V3x2 a, V3x2 b, f2 one) {
   return add_p2(mul2(a.z, b.z), add_p2(mul2(a.x, b.x), mul2(a.y, b.y), one), one);
 }
-// devmath.cuh's fdot and fcross in both lanes (na = -a: the packed forms have
-// no negated operands)
+// devmath.cuh's fdot and cross in both lanes
 __device__ __forceinline__ f2 fdot3(V3x2 a, V3x2 b) { return fma2(a.z, b.z, fma2(a.y, b.y, mul2(a.x, b.x))); }
-__device__ __forceinline__ V3x2 fcross3(V3x2 a, V3x2 na, V3x2 b) {
-  return {fma2(a.y, b.z, mul2(na.z, b.y)), fma2(a.z, b.x, mul2(na.x, b.z)), fma2(a.x, b.y, mul2(na.y, b.x))};
+__device__ __forceinline__ V3x2 cross3(V3x2 a, V3x2 b, f2 one) {
+  return {rsub_p2(mul2(a.z, b.y), mul2(a.y, b.z), one), rsub_p2(mul2(a.x, b.z), mul2(a.z, b.x), one),
+          rsub_p2(mul2(a.y, b.x), mul2(a.x, b.y), one)};
 }
 
 // lane 0 of a where l0, lane 1 of a where l1, the rest of b

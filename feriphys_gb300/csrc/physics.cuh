@@ -30,19 +30,19 @@ __device__ __forceinline__ void strut_forces(V3<T> p0, V3<T> p1, V3<T> v0, V3<T>
 // drag + lift of one face (springy_mesh.rs:634-646): with the face's area A,
 // unit normal n and e = A |n . rv| the reference's
 // -Cd e rv - Cl e |n x rv| rv as one factor times rv, the mean velocity as the
-// sum times RN(1/3) where the reference divides by 3, and sums of products
-// fused.  Fewer roundings than the reference's sequence, in the face terms only.
+// sum times RN(1/3) where the reference divides by 3, and dot products fused.
+// Fewer roundings than the reference's sequence, in the face terms only.
 template <class T>
 __device__ __forceinline__ V3<T> face_total_force(V3<T> x0, V3<T> x1, V3<T> x2, V3<T> v0, V3<T> v1, V3<T> v2,
                                                   V3<T> wind, T neg_cd, T neg_cl) {
   const V3<T> sum = (v0 + v1) + v2;
   const T r3 = sizeof(T) == 8 ? T(1.0 / 3.0) : T(kRcp3);
   const V3<T> rv{fused(sum.x, r3, -wind.x), fused(sum.y, r3, -wind.y), fused(sum.z, r3, -wind.z)};
-  const V3<T> cr = fcross(x1 - x0, x2 - x0);
+  const V3<T> cr = normal_cross(x1 - x0, x2 - x0);
   const T mag = sq_root(fdot(cr, cr));
   const V3<T> n = cr * inv_magnitude(mag);
   const T eff = (mag * T(0.5)) * abs_val(fdot(n, rv));
-  const V3<T> nr = fcross(n, rv);
+  const V3<T> nr = face_cross(n, rv);
   return (eff * fused(neg_cl, sq_root(fdot(nr, nr)), neg_cd)) * rv;
 }
 
@@ -61,7 +61,7 @@ __device__ __forceinline__ T corner_share(V3<T> x0, V3<T> x1, V3<T> x2, T y, int
 }
 template <class T>
 __device__ __forceinline__ T face_corner_weight(V3<T> x0, V3<T> x1, V3<T> x2, int k) {
-  const V3<T> cr = fcross(x1 - x0, x2 - x0);
+  const V3<T> cr = face_cross(x1 - x0, x2 - x0);
   const T y = sq_root(fdot(cr, cr));
   if (sizeof(T) == 8 || k < 2) return corner_share(x0, x1, x2, y, k);
   return (T(1) - corner_share(x0, x1, x2, y, 0)) - corner_share(x0, x1, x2, y, 1);

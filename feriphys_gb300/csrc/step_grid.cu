@@ -273,7 +273,7 @@ __device__ __forceinline__ uint32_t quad_pair(const QuadTerms<TH>& out, int q, c
   for (int k = 0; k < 2; ++k) {
     const PairState &s1 = k ? s11 : s10, &s2 = k ? s10 : s00;
     const FacePair f[1] = {
-        face_pair<FAST>(s01.p, s1.p, s2.p, s01.v, s1.v, s2.v, nwind, neg_cd, neg_lift, far)};
+        face_pair<FAST>(s01.p, s1.p, s2.p, s01.v, s1.v, s2.v, nwind, neg_cd, neg_lift, one, far)};
     f2 w0[1], w1[1];
     face_shares<FAST>(f, one, w0, w1, far);
     V3x2 D = f[0].D;
