@@ -322,8 +322,10 @@ __global__ void __launch_bounds__(32) k_terms64(const Dbl4* pos, const Dbl4* vel
 
 // The sums and the integration are the same for each component, so a vertex
 // has three threads, in three warps; only the collisions, where there are
-// obstacles, take one.
-__global__ void __launch_bounds__(96) k_gather64(int n, const double* pos, const double* vel, const double* force_in,
+// obstacles, take one.  At most 112 registers, six blocks an SM: the unfused
+// collision search takes 118 if it may (90 x 61 tube: 20.1 us a step, 17.7 so;
+// other sizes within 2%).
+__global__ void __maxnreg__(112) k_gather64(int n, const double* pos, const double* vel, const double* force_in,
                                                  double* pos_out, double* vel_out, GeneralTopo t, StepConsts c) {
   __shared__ double sh[9][32];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
