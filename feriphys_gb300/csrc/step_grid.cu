@@ -220,6 +220,10 @@ __device__ __forceinline__ PairState pair_at(const StagedState<TH>& state, int i
   return a;
 }
 
+// Sum of the components' magnitudes, wind's included, below 2^61; false for a NaN.
+__device__ __forceinline__ float length1(V3<float> v) { return fabsf(v.x) + fabsf(v.y) + fabsf(v.z); }
+__device__ __forceinline__ bool mild(V3<float> v, float wind1) { return isfinite((length1(v) + wind1) * 0x1p67f); }
+
 // Where a boundary tile's staged points outside the cloth are put: far away, at
 // rest and no two in the same place.  A strut that does not exist then has
 // some finite length, its constants are zero, and so are its forces; a quad
@@ -227,8 +231,11 @@ __device__ __forceinline__ PairState pair_at(const StagedState<TH>& state, int i
 // Adding a zero of either sign leaves a force sum as it is (no sum is ever -0:
 // it starts from 0 + gravity), so the terms and their sums need no look at
 // what exists, and boundary and interior tiles run the same instructions.  A
-// boundary tile with a non-finite staged state, where zero constants do not
-// make a zero force, takes the slow form of its terms, which does look.
+// boundary tile with a non-finite staged position, or with a velocity or wind
+// that is not `mild`, takes the slow form of its terms, which does look: there
+// a zero constant does not always make a zero force, since a term may overflow
+// before it is multiplied by it.  (Lengths and cross products are 2^50 at most,
+// root_range; times a mild relative velocity they stay below 2^113.)
 // (With a second, checked form of the whole tile beside the unchecked one the
 // two did not fit the instruction cache: 256 cloths of 16..128 vertices a
 // side, which mix both, took 115 instead of 105 us a step.)
@@ -575,7 +582,8 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
 
   // ---- stage the state as pairs: whole rows of EC pairs a round, so a thread
   // keeps its column
-  bool slow = false;  // an edge tile with a non-finite state
+  const float wind1 = length1(wind);
+  bool slow = false;  // an edge tile that looks at what exists
   {
     constexpr int RPR = T::NT / T::EC, ROUNDS = (T::EH + RPR - 1) / RPR;
     const int sr = tid / T::EC, sc = tid - sr * T::EC;
@@ -598,7 +606,7 @@ __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int 
             P[k][l] = state_at(src_p + (k * RPR * C + l * kPairW));
             V[k][l] = state_at(src_v + (k * RPR * C + l * kPairW));
           }
-          slow |= !(finite3(xyz<float>(P[k][l])) && finite3(xyz<float>(V[k][l])));
+          slow |= !(finite3(xyz<float>(P[k][l])) && mild(xyz<float>(V[k][l]), wind1));
         }
       }
     } else {
