@@ -154,7 +154,7 @@ template <class T> constexpr int kStepBlock = sizeof(T) == 4 ? 256 : 32;
 template <class T, int FORM>
 __global__ void __launch_bounds__(kStepBlock<T>, sizeof(T) == 4 ? 4 : 1)
     k_step_general(int n, const Vec4<T>* pos, const Vec4<T>* vel,
-                   const Vec4<T>* __restrict__ force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
+                   const Vec4<T>* force_in, Vec4<T>* __restrict__ pos_out, Vec4<T>* __restrict__ vel_out,
                    GeneralTopo t, StepConsts c) {
   chain_wait();
   chain_next();
@@ -195,7 +195,7 @@ constexpr int kSplitFaceWarps = 3, kSplitFacesEach = 2;
 
 template <int FORM>
 __global__ void __launch_bounds__(32 * (kSplitFaceWarps + 1))
-    k_step_split(int n, const float4* pos, const float4* vel, const float4* __restrict__ force_in,
+    k_step_split(int n, const float4* pos, const float4* vel, const float4* force_in,
                  float4* __restrict__ pos_out, float4* __restrict__ vel_out,
                  GeneralTopo t, StepConsts c) {
   using T = float;

@@ -509,7 +509,7 @@ __host__ __device__ __forceinline__ bool grid_tile(const TileSplit& t, int n_rin
 template <int TH, bool BATCH>
 __device__ __forceinline__ void tile_step(int bx, int by, bool edge, int R, int C, const float* __restrict__ params,
                                           const float4* pos, const float4* vel,
-                                          const float4* __restrict__ force_in, float4* __restrict__ pos_out,
+                                          const float4* force_in, float4* __restrict__ pos_out,
                                           float4* __restrict__ vel_out, const StepConsts& c, V3<float> wind,
                                           unsigned* flags) {
   using T = Tile<TH>;
@@ -822,7 +822,7 @@ template <int TH>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_CTAS)
     k_step_grid_tiled(int R, int C, TileSplit split, int n_ring, const float* __restrict__ params,
                       const float4* pos, const float4* vel,
-                      const float4* __restrict__ force_in, float4* __restrict__ pos_out,
+                      const float4* force_in, float4* __restrict__ pos_out,
                       float4* __restrict__ vel_out, const __grid_constant__ StepConsts c) {
   int bx, by;
   const V3<float> wind{c.wind[0], c.wind[1], c.wind[2]};
