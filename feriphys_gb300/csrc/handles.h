@@ -69,7 +69,7 @@ struct fgb_mesh {
   bool staged = false;
   float* d_io = nullptr;  // as_state staging (10 floats per point; doubles for f64 readback)
   size_t d_io_bytes = 0;
-  float* h_io = nullptr;  // pinned rows for small reads into pageable memory
+  bool pooled_reads = false;  // counts among the users of the pinned rows (capi.cu: RowPool)
   uint8_t* d_pinned = nullptr;
   unsigned* d_flags = nullptr;
 
