@@ -414,7 +414,7 @@ int decide_path(fgb_mesh* m, int* path) {
 }
 
 // The FP64 step's scratch and the struts' points; without room for them the
-// step does without.
+// step does without, as on path 4.
 int ensure_terms64(fgb_mesh* m) {
   const size_t faces = m->topo.fv.size() / 3, struts = m->topo.sa.size();
   if (dalloc(m->d_strut_term, 48 * struts) != cudaSuccess || dalloc(m->d_face_term, 48 * faces) != cudaSuccess ||
@@ -442,7 +442,7 @@ int ensure_topology(fgb_mesh* m) {
     FGB_CUDA(cudaMemcpy(m->d_grid, params.data(), params.size() * sizeof(float), cudaMemcpyHostToDevice));
   } else {
     FGB_CHECK_RC(ensure_csr(m));
-    if (m->precision == 64) FGB_CHECK_RC(ensure_terms64(m));
+    if (m->precision == 64 && !m->plain_csr) FGB_CHECK_RC(ensure_terms64(m));
   }
   m->topo_dirty = false;
   return FGB_OK;

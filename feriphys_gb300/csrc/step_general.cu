@@ -146,8 +146,8 @@ __device__ __forceinline__ void flag_nonfinite(bool bad, unsigned* flags) {
 // Fused Simulation::step for one mesh (accumulate -> integrate -> collide ->
 // pin restore -> clear), one thread per vertex.  The f32 form asks for 4
 // blocks of 256 per SM (at most 64 registers: the gather is latency-bound, so
-// resident warps count).  FP64 comes here only without room for k_terms64's
-// scratch; bound by the FP64 units (one warp instruction takes one of them 64
+// resident warps count).  FP64 comes here, over the plain lists, on path 4 and
+// without room for k_terms64's scratch; bound by the FP64 units (one warp instruction takes one of them 64
 // cycles), it takes single-warp blocks so that a mesh reaches as many of them
 // as it has warps (90 x 61 tube: 123 us a step with blocks of 256, 64 with 32).
 template <class T> constexpr int kStepBlock = sizeof(T) == 4 ? 256 : 32;
@@ -479,15 +479,14 @@ cudaError_t launch_step_general(int n, const void* pos, const void* vel, const v
   // vertex against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3,
   // 360 x 280 14.4 -> 18.6; with launches chained 6.2, 6.4 and, unsplit, 13.9).
   constexpr int kSplitMost = 32768;
-  if constexpr (sizeof(T) == 4) {
-    if (n <= kSplitMost) {
-      run(t.form == 2 ? k_step_split<2> : (t.form == 1 ? k_step_split<1> : k_step_split<0>), blocks_for(n, 32),
-          32 * (kSplitFaceWarps + 1));
-      return cudaGetLastError();
-    }
-  }
-  run(t.form == 2 ? k_step_general<T, 2> : (t.form == 1 ? k_step_general<T, 1> : k_step_general<T, 0>),
-      blocks_for(n, kStepBlock<T>), kStepBlock<T>);
+  if constexpr (sizeof(T) == 8)
+    run(k_step_general<double, 0>, blocks_for(n, kStepBlock<T>), kStepBlock<T>);
+  else if (n <= kSplitMost)
+    run(t.form == 2 ? k_step_split<2> : (t.form == 1 ? k_step_split<1> : k_step_split<0>), blocks_for(n, 32),
+        32 * (kSplitFaceWarps + 1));
+  else
+    run(t.form == 2 ? k_step_general<T, 2> : (t.form == 1 ? k_step_general<T, 1> : k_step_general<T, 0>),
+        blocks_for(n, kStepBlock<T>), kStepBlock<T>);
   return cudaGetLastError();
 }
 

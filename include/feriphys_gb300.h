@@ -165,7 +165,8 @@ int fgb_mesh_export_indices(fgb_mesh* m, void* device_out, void* stream);
  * 3 = the grid kernel's untiled form (one thread per vertex, no shared
  * memory; a cross-check of the tiled one), 4 = the general gather over its
  * plain incidence lists (a cross-check of the compact lists path 1 reads
- * when the mesh fits them).  All give identical results; fgb_mesh_get_path
+ * when the mesh fits them; at precision 64 also vertex by vertex, without the
+ * scratch path 1 keeps its terms in).  All give identical results; fgb_mesh_get_path
  * reports 4 as 1. */
 int fgb_mesh_set_path(fgb_mesh* m, int path);
 
