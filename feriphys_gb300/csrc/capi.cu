@@ -509,10 +509,10 @@ int step_mesh(fgb_mesh* m, const fgb::StepConsts& c) {
     const fgb::GeneralTopo t = general_topo(m);
     if (m->precision == 64)
       FGB_CUDA(fgb::launch_step_general<double>(n, m->pos[m->cur], m->vel[m->cur], F, m->pos[nxt], m->vel[nxt], t,
-                                                c, m->stream, true));
+                                                c, m->stream));
     else
       FGB_CUDA(fgb::launch_step_general<float>(n, m->pos[m->cur], m->vel[m->cur], F, m->pos[nxt], m->vel[nxt], t,
-                                               c, m->stream, true));
+                                               c, m->stream));
   }
   m->cur = nxt;
   m->has_force = false;  // clear_forces

@@ -5,8 +5,8 @@
 // Vector3::angle(a, b) = atan2(|a x b|, a . b).  The library is compiled with
 // -fmad=false so no a*b+c is fused, and '/' and sqrt are the IEEE-rounded
 // operations; with the same operation order the results are bit-identical to
-// the reference's f32 arithmetic except in the face terms: sums of products
-// are fused, drag and lift are one factor of the relative velocity, the atan2
+// the reference's f32 arithmetic except in the face terms: dot products are
+// fused, drag and lift are one factor of the relative velocity, the atan2
 // is the library's own (angle.cuh), and the three corners share one
 // cross-product magnitude (physics.cuh: face_total_force, face_corner_weight).
 #pragma once

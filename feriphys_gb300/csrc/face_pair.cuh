@@ -69,7 +69,8 @@ __device__ __forceinline__ f2 face_last_share(f2 w0, f2 w1, f2 mone) {
   return fma2(w1, mone, fma2(w0, mone, dup2(1.0f)));
 }
 
-// The same with both lanes' results as scalars: D and w0, then w1 and w2.
+// The same with both lanes' results as scalars: D and w0, then w1 and w2 (the
+// form the tests compare with the scalar functions).
 __device__ __forceinline__ void face_terms2(V3x2 x0, V3x2 x1, V3x2 x2, V3x2 v0, V3x2 v1, V3x2 v2, V3x2 wind,
                                             float neg_cd, float neg_lift, float one_rt, float4& DwA, float2& wA,
                                             float4& DwB, float2& wB) {

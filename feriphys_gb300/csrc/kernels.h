@@ -43,10 +43,10 @@ struct GridTopo {
   int variant;  // 0: shared-memory tiles, 1: one thread per vertex reading global memory
 };
 
+// Chained to the launch before it in the stream (chain_launch.cuh).
 template <class T>
 cudaError_t launch_step_general(int n, const void* pos, const void* vel, const void* force_in, void* pos_out,
-                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s,
-                                bool chained);
+                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s);
 template <class T>
 cudaError_t launch_accumulate(int n, const void* pos, const void* vel, void* force, const GeneralTopo& t,
                               const StepConsts& c, cudaStream_t s);

@@ -63,13 +63,12 @@ __device__ __forceinline__ f2 rcp_of_root2(f2 x) {
 
 // The square root of both lanes, exactly the IEEE one, for 2^-100 <= x <=
 // 2^100 (root_range): g = x y and h = y / 2 from the hardware's approximate
-// y = 1/sqrt(x), then the one Newton correction g + h (x - g g) with the
-// residual and the sum fused (the correction step of Markstein's square root,
-// cited in fastdiv.cuh).  Before its last rounding the result is off by about
-// 2^-44 relative; that it then rounds to sqrtf(x) for every float of that
-// range is established by exhaustion (tests/test_gpu_pair.py).  Four packed
-// operations and two approximations for two roots; sqrtf is about ten
-// instructions each, with a range branch.
+// y = 1/sqrt(x), then one step of Newton's iteration for the root of g^2 = x,
+// g + (x - g^2) / (2 sqrt(x)) = g + h (x - g g), with the residual and the sum
+// fused.  Before its last rounding the result is off by about 2^-44 relative;
+// that it then rounds to sqrtf(x) for every float of that range is established
+// by exhaustion (tests/test_gpu_pair.py).  Four packed operations and two
+// approximations for two roots, and no branch.
 constexpr uint32_t kRootLo = 0x0d800000u, kRootSpan = 0x71800000u - 0x0d800000u;  // 2^-100 .. 2^100
 __device__ __forceinline__ float rsqrt_approx_ftz(float x) {
   float r;

@@ -34,6 +34,21 @@ struct PerDeviceOnce {
   }
 };
 
+// SMs of the current device, asked of the driver once for each of the first 64.
+inline int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) {
+    if (dev >= 0 && dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) {
+      if (dev >= 0 && dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+      return sms;
+    }
+  }
+  cudaGetLastError();
+  return 1;
+}
+
 // Restores the calling thread's current device when it goes out of scope.
 class DeviceGuard {
  public:

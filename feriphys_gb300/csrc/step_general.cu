@@ -274,9 +274,10 @@ __global__ void __launch_bounds__(32 * (kSplitFaceWarps + 1))
 // little beside them.  Blocks of the terms are single warps, the long ones
 // first, so that a small mesh reaches every unit.  A face has four threads
 // (its force, and each corner's share, which needs the cross product again) up
-// to kWholeFaces and one beyond, where the units are full anyway (us a step,
-// four and one: 10,800 faces 17.5 and 18.4, 42,000 40 and 67, 60,000 59 and
-// 60, 120,000 104 and 94, 240,000 197 and 168).
+// to kWholeFaces and one beyond, where the units are full (us a step, four and
+// one: 10,700 faces 17.5 and 18.0, 41,800 39.3 and 66.2, 47,800 43.5 and
+// 66.4, 59,700 58.5 and 60.9, 71,800 66 and 75, 89,700 78 and 76, 119,600 104 and
+// 92, 239,400 197 and 172).
 constexpr int kWholeFaces = 65536;
 
 template <int ROLES>
@@ -449,35 +450,34 @@ inline int blocks_for(int n, int bs) { return (n + bs - 1) / bs; }
 
 template <class T>
 cudaError_t launch_step_general(int n, const void* pos, const void* vel, const void* force_in, void* pos_out,
-                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s,
-                                bool chained) {
+                                void* vel_out, const GeneralTopo& t, const StepConsts& c, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const auto run = [&](auto kernel, int blocks, int threads) {
-    chain_launch(kernel, blocks, threads, 0, s, chained, n, static_cast<const Vec4<T>*>(pos),
+    chain_launch(kernel, blocks, threads, 0, s, true, n, static_cast<const Vec4<T>*>(pos),
                  static_cast<const Vec4<T>*>(vel), static_cast<const Vec4<T>*>(force_in),
                  static_cast<Vec4<T>*>(pos_out), static_cast<Vec4<T>*>(vel_out), t, c);
   };
   if constexpr (sizeof(T) == 8) {
-    // (90 x 61 tube: 29.4 us a step in one launch, 17.5 in two; 12 x 10: 24 and 12; 300 x 200: 161 and 94)
+    // (90 x 61 tube: 29.4 us a step in one launch, 17.6 in two; 12 x 10: 24 and 11.4; 300 x 200: 161 and 92.4)
     if (t.strut_term && t.face_term) {
       const bool whole = t.n_faces > kWholeFaces;
       const int terms = (whole ? 1 : 4) * blocks_for(t.n_faces, 32) + blocks_for(t.n_struts, 32);
       if (terms > 0) {
-        const cudaError_t e = chain_launch(whole ? k_terms64<1> : k_terms64<4>, terms, 32, 0, s, chained, static_cast<const Dbl4*>(pos),
-                                           static_cast<const Dbl4*>(vel), t, c);
+        const cudaError_t e = chain_launch(whole ? k_terms64<1> : k_terms64<4>, terms, 32, 0, s, true,
+                                           static_cast<const Dbl4*>(pos), static_cast<const Dbl4*>(vel), t, c);
         if (e != cudaSuccess) return e;
       }
-      return chain_launch(k_gather64, blocks_for(n, 32), 96, 0, s, chained || terms > 0, n,
+      return chain_launch(k_gather64, blocks_for(n, 32), 96, 0, s, true, n,
                           static_cast<const double*>(pos), static_cast<const double*>(vel),
                           static_cast<const double*>(force_in), static_cast<double*>(pos_out),
                           static_cast<double*>(vel_out), t, c);
     }
   }
   // f32: up to this many vertices a step takes as long as one vertex's chain
-  // of terms, which the split kernel shortens; beyond, the SMs are full and
-  // its shared-memory exchange only costs (tubes, us a step, one thread per
-  // vertex against split: 12 x 10 10.4 -> 8.3, 200 x 150 10.4 -> 8.3,
-  // 360 x 280 14.4 -> 18.6; with launches chained 6.2, 6.4 and, unsplit, 13.9).
+  // of terms, which the split kernel shortens; beyond, its shared-memory exchange
+  // only costs (tubes, us a step, one thread per vertex and split: 120 vertices
+  // 7.8 and 5.6, 8,000 7.9 and 6.4, 32,600 8.4 and 6.5, 32,768 7.8 and 6.6; 37,500
+  // 8.4 and 10.6, 60,000 9.6 and 11.6, 100,800 13.8 and 16.4).
   constexpr int kSplitMost = 32768;
   if constexpr (sizeof(T) == 8)
     run(k_step_general<double, 0>, blocks_for(n, kStepBlock<T>), kStepBlock<T>);
@@ -531,7 +531,7 @@ cudaError_t launch_zero4(int n, void* a, cudaStream_t s) {
 
 #define FGB_INSTANTIATE(T)                                                                                        \
   template cudaError_t launch_step_general<T>(int, const void*, const void*, const void*, void*, void*,          \
-                                              const GeneralTopo&, const StepConsts&, cudaStream_t, bool);         \
+                                              const GeneralTopo&, const StepConsts&, cudaStream_t);                     \
   template cudaError_t launch_accumulate<T>(int, const void*, const void*, void*, const GeneralTopo&,            \
                                             const StepConsts&, cudaStream_t);                                     \
   template cudaError_t launch_integrate<T>(int, int, float, const void*, const void*, const void*, void*, void*, \

@@ -974,9 +974,9 @@ cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4*
     if (ea != cudaSuccess) return ea;
     // 8-row tiles, or 4-row ones where there would be no more 8-row tiles than
     // SMs: a tile's latency is the step's then, and the shorter tile has less
-    // (157 x 211: 8.2 us a step with 8 rows, 6.2 with 4; 256 x 256, 256
-    // tiles of 8 rows: 8.2 us either way; 1024 x 1024: 53 us against 61)
-    constexpr int kSms = 152;
+    // (us a step with 8 rows and with 4: 20 x 20 3.82 and 3.53, 64 x 64 4.15 and
+    // 3.78, 157 x 211 4.46 and 4.45; 190 x 200, 168 tiles of 8 rows, 4.73 and
+    // 4.98, 256 x 256 5.8 and 6.1, 1024 x 1024 48 and 56)
     const auto launch = [&](auto kernel, int th, int threads, size_t smem) {
       const TileSplit t = split_tiles(g.rows, g.cols, th);
       const bool has_interior = t.bx1 >= t.bx0 && t.by1 >= t.by0;
@@ -986,7 +986,7 @@ cudaError_t launch_step_grid(const GridTopo& g, const float4* pos, const float4*
                    force_in, pos_out, vel_out, c);
     };
     const long long tiles8 = (long long)((g.cols + kTileW - 1) / kTileW) * ((g.rows + 7) / 8);
-    if (tiles8 <= kSms)
+    if (tiles8 <= sm_count())
       launch(k_step_grid_tiled<4>, 4, Tile<4>::NT, Tile<4>::SMEM);
     else
       launch(k_step_grid_tiled<8>, 8, Tile<8>::NT, Tile<8>::SMEM);

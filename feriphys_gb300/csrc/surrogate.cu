@@ -1347,16 +1347,6 @@ __global__ void k_accept(const float2* __restrict__ cloth_out, int n_cloths, con
   if (c < n_cloths && fail[c]) e_old[c] = cloth_out[c].x;
 }
 
-// SMs of the current device (asked every time: a process may use several devices).
-int sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
-  return sms > 0 ? sms : 1;
-}
-
 template <int G, int H>
 cudaError_t sur_step_attr() {
   // the attribute is per function and per device: set once on each device used

@@ -91,7 +91,7 @@ using Tile = int2;
 // Coarse step of every listed tile: features, MLP on the tensor cores,
 // v' = v + dv, p' = p + (v + v') T / 2 (the mean velocity over the step), collision response against the obstacles
 // (consts: dt = T), pinned vertices unchanged.  groups = 128-thread groups per
-// CTA (2 or 4), ctas = persistent CTAs (0: one per tile group).  stop: a word that
+// CTA (2 or 4), ctas = persistent CTAs at most (0: one per SM); never more than tiles.  stop: a word that
 // turns the launch into one that does nothing when it is not 0 (RolloutCtl), or null.
 cudaError_t launch_sur_step(const SurCloth* cloths, const Tile* tiles, int n_tiles, int parity, const void* blob,
                             const Norm& norm, const StepConsts& consts, int groups, int ctas, int* err,
