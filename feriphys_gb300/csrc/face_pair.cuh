@@ -11,8 +11,8 @@ namespace fgb {
 // Drag + lift of a face (D), and what its corner angles are made of: the
 // cross product's magnitude y and the dot products x0, x1 of corners 0 and 1
 // (springy_mesh.rs:629-654, 134-172), as face_total_force and
-// face_corner_weight compute them.  nwind: the wind negated.  (Every sum of
-// products kept rounded, the drag and the lift apart, took 22 packed
+// face_corner_weight compute them.  nwind: the wind negated.  (Every dot
+// product kept rounded, the drag and the lift apart, took 22 packed
 // operations more per face: 53.2 us a step of the 1024 x 1024 cloth, 51.6
 // with this.)
 struct FacePair {

@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(256) k_step_grid_v1(int R, int C, const float*
 // lanes are paired once, while the state is staged, and never repacked.
 // Measured against one vertex per thread (faces packed only): 1024 x 1024
 // cloth over a plane 57.4 -> 53.8 us a step (43.9 -> 27.7 million warp
-// instructions), 256 cloths of 16..128 vertices a side 133.6 -> 98.7 us (47.6
-// and 94.0 now, with the face terms fused and launches chained).
+// instructions), 256 cloths of 16..128 vertices a side 133.6 -> 98.7 us (48.1
+// and 93.5 now, with the face terms fused and launches chained).
 //
 // The tile and a halo of two vertices (binding struts reach that far) are
 // staged in shared memory as pairs; every strut and face touching the tile is
